@@ -263,6 +263,15 @@ int tci_selftest_bounded_wait(int64_t device, int64_t polls, int64_t* status_out
  * *cycles_per_mma = the slowest SM's clock64 span / (iters x nacc), from the
  * second of two launches. */
 int tci_selftest_mma_rate(int64_t device, int64_t m, int64_t n, int64_t nacc, int64_t iters, double* cycles_per_mma);
+/* The FP64 matrix-instruction GEMM of the device kernels on host arrays:
+ * C (M x N, row pitch ldc) = beta C + alpha sum_{s < nseg} op(A_s) op(B_s),
+ * op(A) M x K (stored K x M when tA), op(B) K x N (stored N x K when tB), row
+ * major with pitches lda, ldb; A_s starts at element a_off + s a_step of the
+ * na-element array A, B_s at b_off + s b_step of the nb-element B. */
+int tci_selftest_gemm_f64(int64_t device, int64_t M, int64_t N, int64_t K, int64_t nseg, int64_t tA, int64_t tB,
+                          int64_t lda, int64_t ldb, int64_t ldc, int64_t a_off, int64_t b_off, int64_t a_step,
+                          int64_t b_step, double alpha, double beta, const double* A, int64_t na, const double* B,
+                          int64_t nb, double* C);
 
 /* ---- A posteriori corrections (calculate_a_posteriori_corrections,
  * tiger_fortran/aposteriori.f90:28-221, called after a one-root SDCI solve,

@@ -1,0 +1,485 @@
+// FP64 grouped GEMM on the double-precision matrix instruction (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind):
+// C (M x N) = beta C + sum over a problem's segments of alpha op(A) op(B), any leading dimension and 8-byte
+// alignment, the problem / segment tables of gemm_tables.h. The instruction is a chain of four fmas in ascending k, so
+// every sum is the one a scalar kernel makes: segments in table order, k ascending, alpha on op(B).
+//
+// Bound by the FP64 pipe: the instruction runs at 37 TFLOP/s on this part, the same as scalar fma, but one operand
+// word read from shared memory feeds eight products instead of four or eight registers' worth of broadcasts, so the
+// pipe, not shared memory or issue slots, sets the rate (the scalar tiled kernels it replaced ran at 10-24 TFLOP/s).
+// Four warps own a 64 x 128 tile, each 64 x 32 of it in 128 accumulator registers, two blocks per SM so that one's
+// copies and barriers run under the other's products; four 16-deep slices in flight by cp.async. Measured on a B200:
+// 592 problems of 256 x 256 x (40 x 256) 30 TFLOP/s, 576 of 173 x 173 x (40 x 173) 20 (6 % of the blocks padding,
+// uneven column shares). Against the scalar kernels: two-external step at 24 pairs x 173 virtuals 102 -> 40 ms, all-
+// external at 240 virtuals 6.8 -> 5.1 ms. Tried and slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp
+// that only copies (registers spill at two blocks per SM), the copies dealt between the products (the loop outgrows
+// the instruction cache: 9-17).
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <stdexcept>
+#include <utility>
+
+#include "../../include/tigerci_sigma.h"
+#include "device_info.h"
+#include "gemm_mma_f64.h"
+
+namespace {
+
+using tci_dev::DGemmProblem;
+using tci_dev::DGemmSeg;
+
+constexpr int NT = 128;  // four warps
+
+__device__ __forceinline__ void cp_async16(unsigned s, const void* g, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async8(unsigned s, const void* g, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void mma884(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};\n"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// Shared-memory layout of an operand slice whose k are contiguous in a row: row r (of the tile) holds BK
+// consecutive k as 16-byte chunks, chunk c at place c ^ swz(r) (within groups of 8).  A fragment read (four rows x
+// four k per half warp) is free of bank conflicts, a transposing copy (consecutive rows, one k) spreads over eight
+// places.  swz moves bits only, so swz(r0 + r1) = swz(r0) ^ swz(r1) where r0 and r1 share no bits.
+__host__ __device__ constexpr int swz(int r) { return ((r & 3) << 1) | ((r >> 2) & 1); }
+// byte offset of chunk c0 + c1 (no common bits, c1 a constant) of a row with swizzle sw
+__device__ __forceinline__ unsigned chunk(int c0, int c1, int sw) {
+  return 16u * (unsigned)(((c0 & ~7) + (c1 & ~7)) | ((c0 & 7) ^ (c1 & 7) ^ sw));
+}
+
+// How an operand reaches shared memory: rows of the tile with k contiguous by 16-byte (K16) or 8-byte (K8) copies,
+// or with the tile rows contiguous: transposed into the row layout by 8-byte copies (RT8, the row operand), or kept
+// as BK rows of the tile rows, pitch R + 2 (R8, R16, the column operand; reads of two k and eight rows spread over
+// the banks).  16-byte copies want a 16-byte aligned operand with an even leading dimension.
+enum Mode { K16, K8, RT8, R8, R16 };
+
+template <int R, int BK, Mode M>
+struct Operand {
+  static constexpr int RP = R <= 8 ? 8 : R <= 16 ? 16 : R <= 32 ? 32 : R <= 64 ? 64 : 128;
+  static constexpr bool KROWS = M == R16, KC = M == K16 || M == K8;
+  static constexpr int PITCH = R + 4;
+  static_assert(!(M == R16) || PITCH % 16 == 4 || PITCH % 16 == 12, "bank spread");
+  static constexpr int SIZE = KROWS ? BK * PITCH : BK * R;  // doubles of a slice
+  // lanes along the contiguous index, rows (of tile or k) a pass, passes
+  static constexpr int LANES = M == K16 ? BK / 2 : M == K8 ? BK : M == R16 ? RP / 2 : RP;
+  static constexpr int PER = NT / LANES, U = KC ? (R + PER - 1) / PER : BK / PER;
+  const double* p;   // this thread's next element
+  long long ustep;   // from one pass to the next
+  int sh = 0;        // R16: the places this thread's rows are shifted by (0 or 1; PER is even)
+  // returns, for R16, the shifts of even (bit 0) and odd (bit 1) k
+  __device__ __forceinline__ int open(const double* X, long long ld, long long row0) {
+    const int x = threadIdx.x % LANES, y = threadIdx.x / LANES;
+    p = X + (KC ? row0 * ld : row0) + (long long)y * ld + (M == K16 || M == R16 ? 2 * x : x);
+    ustep = PER * ld;
+    if constexpr (M == R16) {
+      static_assert(PER % 2 == 0, "a thread's rows have one parity");
+      const int s0 = (int)((reinterpret_cast<uintptr_t>(X + row0) >> 3) & 1), s1 = s0 ^ (int)(ld & 1);
+      sh = (y & 1) ? s1 : s0;
+      p -= sh;
+      return s0 | (s1 << 1);
+    }
+    return 0;
+  }
+  // the slice with min(krem, BK) valid k (zeros past them) into shared memory at s, and on to the next; rows past nr
+  // are left alone: they reach only outputs that are not stored
+  __device__ __forceinline__ void issue(unsigned s, int nr, int krem) {
+    const int x = threadIdx.x % LANES, y = threadIdx.x / LANES;
+    if constexpr (KC) {
+      const int k = M == K16 ? 2 * x : x, sw = swz(y);
+      const int bytes = max(0, min(M == K16 ? 16 : 8, 8 * (krem - k)));
+      if (!bytes) p -= k;  // where nothing is read: an address inside the row (the segment ends here)
+      const unsigned d = s + 8u * (unsigned)(y * BK + (k & 1));
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned o = d + 8u * (u * PER * BK) + chunk(k >> 1, 0, sw ^ swz(u * PER));
+        if (y + u * PER < nr) {
+          if (M == K16) cp_async16(o, p, bytes);
+          else cp_async8(o, p, bytes);
+        }
+        p += ustep;
+      }
+      p += BK - U * ustep;
+    } else {
+      const int r = M == R16 ? 2 * x - sh : x, sw = swz(r);
+      const unsigned d = s + 8u * (unsigned)(KROWS ? y * PITCH + 2 * x : r * BK + (PER > 1 ? (y & 1) : 0));
+      const int bytes = M == RT8 || r + 1 >= nr ? 8 : 16;
+      auto copy = [&](int u, const double* q, int n) {
+        unsigned o;
+        if constexpr (KROWS) o = d + 8u * (u * PER * PITCH);
+        else o = d + (PER > 1 ? chunk(y >> 1, (u * PER) >> 1, sw) : chunk(0, u >> 1, sw) + 8u * (u & 1));
+        if (M == R16) cp_async16(o, q, n);
+        else cp_async8(o, q, n);
+      };
+      if (krem >= BK) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (r < nr) copy(u, p, bytes);
+          p += ustep;
+        }
+      } else {
+        const double* z = p - y * (ustep / PER);  // about the slice's first k, where nothing is read
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const bool ok = y + u * PER < krem;
+          if (r < nr) copy(u, ok ? p : z, ok ? bytes : 0);
+          p += ustep;
+        }
+      }
+    }
+  }
+};
+
+// MB: 8-row blocks of a tile.  WK = 1: the four warps share a tile's columns (up to 16 blocks of 8, dealt evenly),
+// 16-deep k slices; WK = 4: each warp takes a quarter of every 32-deep slice over the whole tile (up to 4 column
+// blocks) and the four sums are added in warp order at the end.  Tiles are cut evenly in 8-row / 8-column blocks (a
+// 173-row problem gives 64 + 56 + 56 rows, not 64 + 64 + 45); blocks past the edge are not computed.
+constexpr int NB = 4;  // column blocks of a warp at most
+template <int MB, int WK, Mode AM, Mode BM_>
+struct Shape {
+  static constexpr int BK = WK == 1 ? 16 : 32;
+  static constexpr int BM = 8 * MB, BN = 8 * NB * (WK == 1 ? 4 : 1);
+  using A = Operand<BM, BK, AM>;
+  using B = Operand<(WK == 4 && BM_ == R16 ? BN + 8 : BN), BK, BM_>;  // room for a shifted row
+  static constexpr int STAGE = A::SIZE + B::SIZE;  // doubles
+  static constexpr int STG = 4;
+  static constexpr size_t smem = sizeof(double) * (size_t)STAGE * STG;
+};
+
+template <int MB, int WK, Mode AM, Mode BM_>
+__global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
+                                                      const DGemmSeg* __restrict__ segs) {
+  using Sh = Shape<MB, WK, AM, BM_>;
+  constexpr int BK = Sh::BK, STG = Sh::STG;
+  constexpr bool KB = Sh::B::KROWS;
+  extern __shared__ __align__(128) double sm[];
+  __shared__ double meta_alpha[STG];
+  __shared__ int meta_k[STG];  // valid k of the slice; + 256: alpha is not 1; + 512, 1024: shifts of even, odd k
+  const int lane = threadIdx.x & 31;
+  // rotated: the uneven shares fall on every scheduler in turn
+  const int role = ((threadIdx.x >> 5) + blockIdx.x) & 3;
+  // the problem of this tile (the last with tile_begin <= tile), 32 probes at a time
+  const long long tile = blockIdx.x;
+  int lo = 0, cnt = nprob;
+  while (cnt > 1) {
+    const int step = (cnt + 31) >> 5, off = lane * step;
+    const bool ok = off < cnt && probs[lo + off].tile_begin <= tile;
+    const int c = 31 - __clz(__ballot_sync(0xffffffffu, ok));
+    lo += c * step;
+    cnt = min(step, cnt - c * step);
+  }
+  const DGemmProblem P = probs[lo];
+  const bool tr = P.trans_c != 0;
+  const long long rows = tr ? P.N : P.M, cols = tr ? P.M : P.N;
+  const int tn = (int)P.tiles_n, t = (int)(tile - P.tile_begin), ti = t / tn, tj = t % tn;
+  const int mblk = (int)((rows + 7) >> 3), nblk = (int)((cols + 7) >> 3), tm = (mblk + 7) >> 3;
+  const int mq = mblk / tm, mr = mblk % tm, nq = nblk / tn, nr = nblk % tn;
+  const long long m0 = 8ll * (ti * mq + min(ti, mr)), n0 = 8ll * (tj * nq + min(tj, nr));
+  const int mb = mq + (ti < mr ? 1 : 0), nbt = nq + (tj < nr ? 1 : 0);  // mb: MB or MB - 1
+  const int mrows = (int)min((long long)(8 * mb), rows - m0), ncols = (int)min((long long)(8 * nbt), cols - n0);
+  // this warp's column blocks of the tile
+  const int j0 = WK == 1 ? (nbt * role) >> 2 : 0, nb = WK == 1 ? ((nbt * (role + 1)) >> 2) - j0 : nbt;
+  const int g = lane >> 2, tq = lane & 3;
+
+  double acc[MB][NB][2];
+#pragma unroll
+  for (int i = 0; i < MB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+  // the slices of all segments in table order, copied STG - 1 ahead
+  const unsigned sbase = static_cast<unsigned>(__cvta_generic_to_shared(sm));
+  int sg = (int)P.seg_begin;
+  const int sge = (int)P.seg_end;
+  int krem = 0, flags = 0;
+  double alpha = 1.0;
+  typename Sh::A oa;
+  typename Sh::B ob;
+  DGemmSeg S{};
+  if (sg < sge) S = segs[sg];
+  auto open = [&]() {  // segment sg (loaded earlier), and the load of the one after it
+    krem = (int)S.K;
+    alpha = S.alpha;
+    oa.open(tr ? S.B : S.A, tr ? S.ldb : S.lda, m0);
+    flags = 512 * ob.open(tr ? S.A : S.B, tr ? S.lda : S.ldb, n0) + (alpha != 1.0 ? 256 : 0);
+    if (sg + 1 < sge) S = segs[sg + 1];
+  };
+  if (sg < sge) open();
+  auto produce = [&](int st) {
+    if (krem > 0) {
+      const unsigned s = sbase + 8u * (unsigned)(st * Sh::STAGE);
+      oa.issue(s, mrows, krem);
+      ob.issue(s + 8u * (unsigned)Sh::A::SIZE, ncols, krem);
+      if (threadIdx.x == 0) {
+        meta_alpha[st] = alpha;
+        meta_k[st] = min(BK, krem) + flags;
+      }
+      krem -= BK;
+      if (krem <= 0 && ++sg < sge) open();
+    } else if (threadIdx.x == 0) {
+      meta_k[st] = 0;
+    }
+    cp_commit();
+  };
+#pragma unroll 1
+  for (int st = 0; st < STG - 1; ++st) produce(st);
+  // fragment addresses: lane (g, tq) holds row g of a block at k = 4 s + tq of step s; with k contiguous, step s's
+  // chunks 2 s, 2 s + 1 of a row's 8
+  const int f0 = g * BK + 2 * ((tq >> 1) ^ swz(g)) + (tq & 1);
+  const int bo = Sh::A::SIZE + (KB ? j0 * 8 + tq * Sh::B::PITCH + g : j0 * 8 * BK);
+  int st = 0;
+  for (;;) {
+    cp_wait<STG - 2>();  // this thread's copies of the slice have landed
+    __syncthreads();     // everyone's have, and the stage refilled below is no longer read
+    const int mk = meta_k[st];
+    if (mk == 0) break;
+    const int kc = mk & 255;
+    const double al = meta_alpha[st];
+    produce(st == 0 ? STG - 1 : st - 1);
+    const double* as = sm + st * Sh::STAGE;
+    const double* bs = as + bo + (KB ? (mk >> (9 + (tq & 1))) & 1 : 0);
+    auto step = [&](int s4) {  // four k
+      const int fo = (f0 ^ ((s4 & 3) << 2)) + (s4 >> 2) * 16;
+      double a[MB];
+#pragma unroll
+      for (int i = 0; i < MB; ++i) a[i] = as[i * 8 * BK + fo];
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        if (j >= nb) break;
+        double b = KB ? bs[s4 * 4 * Sh::B::PITCH + j * 8] : bs[j * 8 * BK + fo];
+        if (mk & 256) b *= al;
+#pragma unroll
+        for (int i = 0; i < MB - 1; ++i) mma884(acc[i][j][0], acc[i][j][1], a[i], b);
+        if (mb == MB) mma884(acc[MB - 1][j][0], acc[MB - 1][j][1], a[MB - 1], b);
+      }
+    };
+    if constexpr (WK == 1) {
+#pragma unroll
+      for (int s4 = 0; s4 < BK / 4; ++s4)
+        if (4 * s4 < kc) step(s4);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (8 * role + 4 * q < kc) step(2 * role + q);
+    }
+    st = st == STG - 1 ? 0 : st + 1;
+  }
+  cp_wait<0>();
+  auto store = [&](int i, int j, double v0, double v1) {
+    const long long r = m0 + 8 * i + g, c = n0 + 8 * (j0 + j) + 2 * tq;
+    if (r >= rows) return;
+    double* x = P.C + (tr ? c * P.ldc + r : r * P.ldc + c);
+    const long long d = tr ? P.ldc : 1;
+    if (c < cols) x[0] = P.beta == 0.0 ? v0 : fma(P.beta, x[0], v0);
+    if (c + 1 < cols) x[d] = P.beta == 0.0 ? v1 : fma(P.beta, x[d], v1);
+  };
+  if constexpr (WK == 1) {
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j < nb) {
+#pragma unroll
+        for (int i = 0; i < MB; ++i)
+          if (i < mb) store(i, j, acc[i][j][0], acc[i][j][1]);
+      }
+  } else {
+    __syncthreads();  // the stages are free
+    double2* red = reinterpret_cast<double2*>(sm);
+#pragma unroll
+    for (int i = 0; i < MB; ++i)
+#pragma unroll
+      for (int j = 0; j < NB; ++j) red[(role * MB * NB + i * NB + j) * 32 + lane] = make_double2(acc[i][j][0], acc[i][j][1]);
+    __syncthreads();
+    for (int e = role; e < MB * NB; e += 4) {
+      const int i = e / NB, j = e % NB;
+      if (i >= mb || j >= nb) continue;
+      double2 v = red[e * 32 + lane];
+#pragma unroll
+      for (int w = 1; w < 4; ++w) {
+        const double2 x = red[(w * MB * NB + e) * 32 + lane];
+        v.x += x.x;
+        v.y += x.y;
+      }
+      store(i, j, v.x, v.y);
+    }
+  }
+}
+
+template <int MB, int WK, Mode AM, Mode BM_>
+cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles, cudaStream_t st) {
+  constexpr size_t smem = Shape<MB, WK, AM, BM_>::smem;
+  static_assert(WK == 1 || smem >= sizeof(double2) * 4 * MB * NB * 32, "the warps' sums fit the stages");
+  static std::once_flag once[64];  // the attribute, once per device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::call_once(once[dev], [&] {
+    cudaFuncSetAttribute(gemm_mma_f64<MB, WK, AM, BM_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  gemm_mma_f64<MB, WK, AM, BM_><<<(unsigned)ntiles, NT, smem, st>>>(probs, nprob, segs);
+  return cudaGetLastError();
+}
+
+using Go = cudaError_t (*)(const DGemmProblem*, int, const DGemmSeg*, long long, cudaStream_t);
+#define TCI_ROWS(WK, A, B) \
+  go<1, WK, A, B>, go<2, WK, A, B>, go<3, WK, A, B>, go<4, WK, A, B>, go<5, WK, A, B>, go<6, WK, A, B>, go<7, WK, A, B>, \
+      go<8, WK, A, B>
+#define TCI_PAIR(A, B) TCI_ROWS(1, A, B), TCI_ROWS(4, A, B)
+constexpr Go kGo[tci_dmma::CLASSES] = {TCI_PAIR(K16, K16), TCI_PAIR(K16, R16), TCI_PAIR(K8, K8),
+                                       TCI_PAIR(K8, R16),  TCI_PAIR(RT8, K8),  TCI_PAIR(RT8, R16)};
+#undef TCI_PAIR
+#undef TCI_ROWS
+
+// Tile counts of a problem of rows x cols: at most 8 row blocks x bnb column blocks (the warps sharing k: 8 x 4).
+struct Cut {
+  long long tm, tn;
+  int mb, nb;   // blocks of its largest tile
+  double cost;  // 8 x 8 blocks computed, each tile's slowest warp times four
+};
+Cut cut(long long rows, long long cols, int bnb) {
+  const long long mblk = (rows + 7) / 8, nblk = (cols + 7) / 8;
+  Cut c;
+  c.tm = (mblk + 7) / 8;
+  c.tn = (nblk + bnb - 1) / bnb;
+  c.mb = (int)((mblk + c.tm - 1) / c.tm);
+  c.nb = (int)((nblk + c.tn - 1) / c.tn);
+  c.cost = (double)mblk * (double)c.tn * (double)(bnb <= NB ? c.nb : (c.nb + 3) / 4 * 4);
+  return c;
+}
+
+// Adds a problem to the class its operands and tile allow; bnb = NB: the warps share k.  *work: the largest tile's
+// blocks x the problem's k.
+void add_problem(const DGemmProblem& g, const std::vector<DGemmSeg>& segs, int bnb, tci_dmma::Tiles& t, double& work) {
+  DGemmProblem x = g;
+  x.trans_c = cut(g.N, g.M, bnb).cost < 0.8 * cut(g.M, g.N, bnb).cost ? 1 : 0;
+  bool row_k = true, row_r = true, col_k = true, col_r = true, row_even = true, col_even = true;
+  double k = 0;
+  for (long long q = g.seg_begin; q < g.seg_end; ++q) {
+    const DGemmSeg& y = segs[(size_t)q];
+    const bool rk = x.trans_c ? y.tB != 0 : y.tA == 0, ck = x.trans_c ? y.tA == 0 : y.tB != 0;
+    row_k = row_k && rk;
+    row_r = row_r && !rk;
+    col_k = col_k && ck;
+    col_r = col_r && !ck;
+    const bool ea = (y.lda & 1) == 0 && (reinterpret_cast<uintptr_t>(y.A) & 15) == 0;
+    const bool eb = (y.ldb & 1) == 0 && (reinterpret_cast<uintptr_t>(y.B) & 15) == 0;
+    row_even = row_even && (x.trans_c ? eb : ea);
+    col_even = col_even && (x.trans_c ? ea : eb);
+    k += (double)y.K;
+  }
+  if ((!row_k && !row_r) || (!col_k && !col_r))
+    throw std::invalid_argument("a GEMM problem whose segments differ in storage order");
+  if (!col_k && !col_even && bnb > NB) bnb = std::min(bnb, 15);  // room for shifted rows
+  const Cut c = x.trans_c ? cut(g.N, g.M, bnb) : cut(g.M, g.N, bnb);
+  const int modes = !row_k ? (col_k ? 4 : 5) : col_k ? (row_even && col_even ? 0 : 2) : (row_even ? 1 : 3);
+  const int cls = c.mb - 1 + (bnb <= NB ? 8 : 0) + 16 * modes;
+  x.tiles_n = c.tn;
+  x.tile_begin = t.ntiles[cls];
+  t.ntiles[cls] += c.tm * c.tn;
+  t.probs[cls].push_back(x);
+  work = std::max(work, (double)c.mb * (bnb <= NB ? c.nb : (c.nb + 3) / 4 * 4) * k);
+}
+
+}  // namespace
+
+namespace tci_dmma {
+
+Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& segs) {
+  // the longest problems first: the short ones fill the last wave
+  std::vector<std::pair<long long, size_t>> order;
+  for (size_t i = 0; i < pr.size(); ++i) {
+    long long k = 0;
+    for (long long q = pr[i].seg_begin; q < pr[i].seg_end; ++q) k += segs[(size_t)q].K;
+    order.push_back({-k, i});
+  }
+  std::stable_sort(order.begin(), order.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+  // Tile width by the time the fullest SM would need: waves of tiles x the largest tile, the narrower ones at the
+  // rate they were measured at (28 TFLOP/s for 12 blocks, 24 for 8 and 19 for the k-sharing 4 against 30 for 16 on
+  // a launch that fills the chip).  Wide tiles win once there are several waves, narrow and k-sharing ones where a
+  // launch would leave SMs idle.
+  const double sms = (double)tci_dev::device_sms();
+  Tiles best;
+  double best_time = 0;
+  for (const auto& [bnb, slow] : {std::pair<int, double>{16, 1.0}, {12, 1.12}, {8, 1.25}, {NB, 1.6}}) {
+    Tiles t;
+    double work = 0, n = 0;
+    for (const auto& o : order) add_problem(pr[o.second], segs, bnb, t, work);
+    for (long long k : t.ntiles) n += (double)k;
+    const double time = std::ceil(n / sms) * work * slow;
+    if (bnb == 16 || time < 0.97 * best_time) {
+      best = std::move(t);
+      best_time = time;
+    }
+    if (n > 16 * sms) break;
+  }
+  return best;
+}
+
+cudaError_t launch(const Tables& t, const DGemmSeg* segs, cudaStream_t st) {
+  for (int c = 0; c < CLASSES; ++c) {
+    if (t.ntiles[c] <= 0) continue;
+    const cudaError_t e = kGo[c](t.probs[c], t.nprob[c], segs, t.ntiles[c], st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace tci_dmma
+
+// Test entry: C (M x N) = beta C + alpha sum_s op(A_s) op(B_s) on host arrays, nseg matrices a_step / b_step apart
+// from element a_off / b_off on.
+extern "C" int tci_selftest_gemm_f64(int64_t device, int64_t M, int64_t N, int64_t K, int64_t nseg, int64_t tA, int64_t tB,
+                                     int64_t lda, int64_t ldb, int64_t ldc, int64_t a_off, int64_t b_off, int64_t a_step,
+                                     int64_t b_step, double alpha, double beta, const double* A, int64_t na,
+                                     const double* B, int64_t nb, double* C) {
+  if (!A || !B || !C || M < 1 || N < 1 || K < 1 || nseg < 0 || a_off < 0 || b_off < 0 || a_step < 0 || b_step < 0 ||
+      lda < (tA ? M : K) || ldb < (tB ? K : N) || ldc < N)
+    return TCI_ERR_ARG;
+  const int64_t ea = ((tA ? K : M) - 1) * lda + (tA ? M : K), eb = ((tB ? N : K) - 1) * ldb + (tB ? K : N);
+  if (nseg > 0 && (a_off + (nseg - 1) * a_step + ea > na || b_off + (nseg - 1) * b_step + eb > nb)) return TCI_ERR_ARG;
+  double *dA = nullptr, *dB = nullptr, *dC = nullptr;
+  DGemmSeg* ds = nullptr;
+  DGemmProblem* dp = nullptr;
+  int rc = TCI_OK;
+  auto ok = [&](cudaError_t e) {
+    if (e != cudaSuccess && rc == TCI_OK) rc = TCI_ERR_CUDA;
+    return rc == TCI_OK;
+  };
+  try {
+    const size_t cb = sizeof(double) * (size_t)((M - 1) * ldc + N);
+    if (ok(cudaSetDevice((int)device)) && ok(cudaMalloc(&dA, sizeof(double) * (size_t)na)) &&
+        ok(cudaMalloc(&dB, sizeof(double) * (size_t)nb)) && ok(cudaMalloc(&dC, cb)) &&
+        ok(cudaMalloc(&ds, sizeof(DGemmSeg) * (size_t)std::max<int64_t>(1, nseg))) && ok(cudaMalloc(&dp, sizeof(DGemmProblem)))) {
+      std::vector<DGemmSeg> segs;
+      for (int64_t q = 0; q < nseg; ++q)
+        segs.push_back(DGemmSeg{dA + a_off + q * a_step, dB + b_off + q * b_step, lda, ldb, K, tA ? 1 : 0, tB ? 1 : 0, alpha});
+      const tci_dmma::Tiles t = tci_dmma::tile({DGemmProblem{dC, ldc, M, N, 0, 0, beta, 0, nseg, 0}}, segs);
+      ok(cudaMemcpy(dA, A, sizeof(double) * (size_t)na, cudaMemcpyHostToDevice));
+      ok(cudaMemcpy(dB, B, sizeof(double) * (size_t)nb, cudaMemcpyHostToDevice));
+      ok(cudaMemcpy(dC, C, cb, cudaMemcpyHostToDevice));
+      if (nseg > 0) ok(cudaMemcpy(ds, segs.data(), sizeof(DGemmSeg) * segs.size(), cudaMemcpyHostToDevice));
+      tci_dmma::Tables d;
+      for (int c = 0; c < tci_dmma::CLASSES; ++c)
+        if (t.ntiles[c] > 0) {
+          ok(cudaMemcpy(dp, t.probs[c].data(), sizeof(DGemmProblem), cudaMemcpyHostToDevice));
+          d.probs[c] = dp;
+          d.nprob[c] = 1;
+          d.ntiles[c] = t.ntiles[c];
+        }
+      if (rc == TCI_OK) ok(tci_dmma::launch(d, ds, 0));
+      ok(cudaDeviceSynchronize());
+      ok(cudaMemcpy(C, dC, cb, cudaMemcpyDeviceToHost));
+    }
+  } catch (...) {
+    rc = TCI_ERR_INTERNAL;
+  }
+  for (void* p : {(void*)dA, (void*)dB, (void*)dC, (void*)ds, (void*)dp}) cudaFree(p);
+  return rc;
+}

@@ -1,0 +1,34 @@
+// FP64 grouped GEMM on the double-precision matrix instruction (gemm_mma_f64.cu): host side.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "gemm_tables.h"
+
+namespace tci_dmma {
+
+// Problems sorted into the kernel's tile classes: the shape of a tile and how its four warps share it (rows and
+// columns, or k slices where a launch has too few tiles) x the two storage orders of the column operand.
+constexpr int CLASSES = 96;
+struct Tiles {
+  std::vector<tci_dev::DGemmProblem> probs[CLASSES];
+  long long ntiles[CLASSES] = {};
+};
+// Sorts a launch's problems (their tiles_n, tile_begin and trans_c are set here).
+Tiles tile(const std::vector<tci_dev::DGemmProblem>& pr, const std::vector<tci_dev::DGemmSeg>& segs);
+// The device copies of a Tiles.
+struct Tables {
+  tci_dev::DGemmProblem* probs[CLASSES] = {};
+  int nprob[CLASSES] = {};
+  long long ntiles[CLASSES] = {};
+  int launches() const {
+    int k = 0;
+    for (long long t : ntiles) k += t > 0 ? 1 : 0;
+    return k;
+  }
+};
+// All classes of a launch, segs the table its problems index.
+cudaError_t launch(const Tables& t, const tci_dev::DGemmSeg* segs, cudaStream_t st);
+
+}  // namespace tci_dmma

@@ -1,5 +1,5 @@
 // Device-side tables of a grouped GEMM (8-byte fields), shared by the FP64
-// SIMT kernel (sigma_device.cu) and the tcgen05 kernel (gemm_tc.cu), and the
+// kernel (gemm_mma_f64.cu) and the tcgen05 kernel (gemm_tc.cu), and the
 // host helper that tiles a list of problems for either kernel.
 //
 //   C (M x N, row pitch ldc) = beta C + sum over the problem's segments of
@@ -17,7 +17,8 @@ struct DGemmProblem {
   long long ldc, M, N, tiles_n, tile_begin;  // tiles_n, tile_begin: in the launching kernel's tile shape
   double beta;
   long long seg_begin, seg_end;
-  long long trans_c;  // tensor-core tables only: M, N and the segments describe C^T = B^T A^T
+  long long trans_c;  // gemm_tc.cu: M, N and the segments describe C^T = B^T A^T;
+                         // gemm_mma_f64.cu: computed with the operands swapped
 };
 struct DGemmSeg {
   const double* A;
@@ -58,17 +59,5 @@ inline long long tile_problems(const std::vector<HostGemm>& in, long long tm, lo
   }
   return tiles;
 }
-
-// FP64 SIMT grouped GEMM (sigma_device.cu); cfg 0: 64 x 128 tiles, 1: 128 x 64.
-cudaError_t launch_gemm_f64(int cfg, const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles,
-                            cudaStream_t st);
-// The cp.async-staged FP64 kernel (64 x 128 tiles): A not transposed, B K x N, operands 16-byte aligned
-// with even leading dimensions.
-cudaError_t launch_gemm_cp_f64(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles,
-                               cudaStream_t st);
-inline long long gemm_cp_tile_m() { return 64; }
-inline long long gemm_cp_tile_n() { return 128; }
-inline long long gemm_f64_tile_m(int cfg) { return cfg == 0 ? 64 : 128; }
-inline long long gemm_f64_tile_n(int cfg) { return cfg == 0 ? 128 : 64; }
 
 }  // namespace tci_dev

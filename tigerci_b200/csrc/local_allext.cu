@@ -56,6 +56,7 @@
 #include "../../include/tigerci_sigma.h"
 #include "allext_tc.h"
 #include "device_info.h"
+#include "gemm_mma_f64.h"
 #include "gemm_tables.h"
 #include "gemm_tma.h"
 #include "host/capi_internal.h"
@@ -261,11 +262,8 @@ __global__ void add_into(double* __restrict__ dst, const double* __restrict__ sr
 }
 
 struct GemmLaunch {
-  DGemmProblem* probs = nullptr;
+  tci_dmma::Tables t;
   DGemmSeg* segs = nullptr;
-  int nprob = 0;
-  long long ntiles = 0;
-  int cfg = 0;  // FP64 tile shape
 };
 struct TmaLaunch {
   TmaProblem* probs = nullptr;
@@ -283,7 +281,7 @@ struct tci_local {
   int64_t npv = 0;   // virtual pairs
   int64_t jmax = 0;  // largest chunk the buffers hold
   int64_t jc = 0;    // chunk in use
-  int cfg2 = 0;      // FP64 tile shape of the second GEMM in use
+  int cfg2 = 0;      // mixed form: tile width of the first GEMM in use (0: 128, 1: 64)
   double flops = 0, lbytes = 0, dev_bytes = 0, last_ms = 0, tuned_ms = 0;
   int64_t candidates = 0;
   std::vector<void*> owned;
@@ -372,7 +370,7 @@ struct tci_local {
   }
 
   // FP64 form: GEMM tables for chunks of j vectors (the chunk buffers are laid out for jmax)
-  void make_gemms(int64_t j, int cfg_second, GemmLaunch& a, GemmLaunch& b) {
+  void make_gemms(int64_t j, GemmLaunch& a, GemmLaunch& b) {
     std::vector<HostGemm> v1, v2;
     for (const auto& B : blocks) {
       const DLocHead& H = heads[B.head];
@@ -384,21 +382,20 @@ struct tci_local {
         y.segs.push_back(DGemmSeg{Tk + q * n * ld, Lc + H.lc_off + q * n * ld, ld, ld, n, 0, 0, 0.5});
       v2.push_back(std::move(y));
     }
-    auto finish = [&](std::vector<HostGemm>& v, int cfg, GemmLaunch& g) {
+    auto finish = [&](std::vector<HostGemm>& v, GemmLaunch& g) {
       std::vector<DGemmProblem> pr;
       std::vector<DGemmSeg> sg;
-      g.cfg = cfg;
-      const long long tm = cfg == 2 ? tci_dev::gemm_cp_tile_m() : tci_dev::gemm_f64_tile_m(cfg);
-      const long long tn = cfg == 2 ? tci_dev::gemm_cp_tile_n() : tci_dev::gemm_f64_tile_n(cfg);
-      g.ntiles = tci_dev::tile_problems(v, tm, tn, false, pr, sg);
-      g.probs = upload(pr);
+      tci_dev::tile_problems(v, 64, 64, false, pr, sg);
+      const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
+      for (int c = 0; c < tci_dmma::CLASSES; ++c) {
+        g.t.probs[c] = upload(t.probs[c]);
+        g.t.nprob[c] = (int)t.probs[c].size();
+        g.t.ntiles[c] = t.ntiles[c];
+      }
       g.segs = upload(sg);
-      g.nprob = (int)pr.size();
     };
-    // cfg_second 0: both GEMMs on the cp.async-staged kernel (64 x 128 tiles; the even row pitches keep every
-    // operand row 16-byte aligned); 1: the register-staged kernel, 128 x 64 tiles
-    finish(v1, cfg_second == 0 ? 2 : 1, a);
-    finish(v2, cfg_second == 0 ? 2 : 1, b);
+    finish(v1, a);
+    finish(v2, b);
   }
 
   // mixed form: TMA-fed tables for chunks of j vectors; narrow1: the first GEMM on 64-wide tiles
@@ -436,9 +433,7 @@ struct tci_local {
   }
 
   void launch_gemm(const GemmLaunch& g) {
-    if (g.ntiles <= 0) return;
-    if (g.cfg == 2) LCUDA(tci_dev::launch_gemm_cp_f64(g.probs, g.nprob, g.segs, g.ntiles, stream));
-    else LCUDA(tci_dev::launch_gemm_f64(g.cfg, g.probs, g.nprob, g.segs, g.ntiles, stream));
+    LCUDA(tci_dmma::launch(g.t, g.segs, stream));
   }
 
   // Dense form set-up from the virtual-virtual Cholesky rows lpk (npv x nchol, row-major, on the device):
@@ -549,7 +544,7 @@ struct tci_local {
     LCUDA(cudaGetLastError());
   }
 
-  // Tables and graph for chunk size j and second-GEMM tile shape cfg (Cholesky form).
+  // Tables and graph for chunk size j and first-GEMM tile width cfg (Cholesky form).
   void configure(int64_t j, int cfg) {
     release_graph();
     form = 0;
@@ -560,8 +555,8 @@ struct tci_local {
       make_tma(jc, cfg2 == 1, m1, m2);
       if (rem) make_tma(rem, cfg2 == 1, m1r, m2r);
     } else {
-      make_gemms(jc, cfg2, g1, g2);
-      if (rem) make_gemms(rem, cfg2, g1r, g2r);
+      make_gemms(jc, g1, g2);
+      if (rem) make_gemms(rem, g1r, g2r);
     }
     capture();
   }
@@ -794,14 +789,14 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
     L->dblocks = L->upload(L->blocks);
     L->ddom = L->upload(dom);
 
-    // autotuner: chunk size (largest, half, quarter) x FP64 tile shape of the second GEMM (mixed form: tile
-    // width of the first GEMM, 128 or 64); one timed run each.  Then the dense form, timed on its second
+    // autotuner: chunk size (largest, half, quarter), in the mixed form x tile width of the first GEMM (128 or
+    // 64); one timed run each.  Then the dense form, timed on its second
     // run; the faster form stays and the other's buffers are released.
     double best = 1e300;
     if (chol_form) {
       std::vector<std::pair<int64_t, int>> cand;
       for (int64_t j : {L->jmax, std::max<int64_t>(1, L->jmax / 2), std::max<int64_t>(1, L->jmax / 4)})
-        for (int cfg : {0, 1}) {
+        for (int cfg = 0; cfg < (L->precision == 1 ? 2 : 1); ++cfg) {
           if (std::find(cand.begin(), cand.end(), std::make_pair(j, cfg)) == cand.end()) cand.push_back({j, cfg});
         }
       if (!tune) cand.resize(1);

@@ -1,8 +1,5 @@
 // Device executor of the sigma plan (host/plan.h) and the device half of the C
-// ABI.  Kernels here (FP64):
-//   gemm_tiled_f64    C = beta*C + sum_seg alpha*op(A)op(B), one CTA per 64x128
-//                     or 128x64 tile of every problem, segments summed in table
-//                     order (split-K for few-tile, long-K steps)
+// ABI.  The FP64 GEMM steps run on gemm_mma_f64.cu; kernels here (FP64):
 //   gemm_skinny_f64   problems of at most 8 rows: a warp per output column
 //   axpy_segments     one block per target chunk, sources summed in table order
 //   dot_segments      one block per target scalar
@@ -33,6 +30,7 @@
 #include "../../include/tigerci_sigma.h"
 #include "allext_tc.h"
 #include "device_info.h"
+#include "gemm_mma_f64.h"
 #include "gemm_tables.h"
 #include "gemm_tc.h"
 #include "gemm_tma.h"
@@ -80,200 +78,6 @@ struct DDotSource {
 struct DHead {
   long long off_ab, off_aa, nsf_ab, nsf_aa, nsing, nD, dk0;
 };
-
-constexpr int GT = 64;   // tile edge
-constexpr int GK = 16;   // k step
-constexpr int GTH = 256; // threads (16 x 16, 4 x 4 outputs each)
-
-__global__ void __launch_bounds__(GTH) gemm_grouped_f64(const DGemmProblem* __restrict__ probs, int nprob,
-                                                        const DGemmSeg* __restrict__ segs) {
-  __shared__ double As[GK][GT + 1];
-  __shared__ double Bs[GK][GT + 1];
-  // locate problem of this tile
-  const long long tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile_begin <= tile) lo = mid;
-    else hi = mid - 1;
-  }
-  const DGemmProblem P = probs[lo];
-  const long long t = tile - P.tile_begin;
-  const long long m0 = (t / P.tiles_n) * GT, n0 = (t % P.tiles_n) * GT;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  for (long long s = P.seg_begin; s < P.seg_end; ++s) {
-    const DGemmSeg S = segs[s];
-    double acs[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acs[i][j] = 0.0;
-    for (long long k0 = 0; k0 < S.K; k0 += GK) {
-      // load A tile (GT rows x GK cols) into As[k][m]
-      for (int e = threadIdx.x; e < GT * GK; e += GTH) {
-        int mm, kk;
-        if (S.tA) { mm = e % GT; kk = e / GT; }   // A stored K x M: contiguous in m
-        else { kk = e % GK; mm = e / GK; }        // A stored M x K: contiguous in k
-        const long long gm = m0 + mm, gk = k0 + kk;
-        double v = 0.0;
-        if (gm < P.M && gk < S.K) v = S.tA ? S.A[gk * S.lda + gm] : S.A[gm * S.lda + gk];
-        As[kk][mm] = v;
-      }
-      for (int e = threadIdx.x; e < GT * GK; e += GTH) {
-        int nn, kk;
-        if (S.tB) { kk = e % GK; nn = e / GK; }   // B stored N x K
-        else { nn = e % GT; kk = e / GT; }        // B stored K x N
-        const long long gn = n0 + nn, gk = k0 + kk;
-        double v = 0.0;
-        if (gn < P.N && gk < S.K) v = S.tB ? S.B[gn * S.ldb + gk] : S.B[gk * S.ldb + gn];
-        Bs[kk][nn] = v;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < GK; ++kk) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acs[i][j] = fma(a[i], b[j], acs[i][j]);
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fma(S.alpha, acs[i][j], acc[i][j]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long gm = m0 + ty + 16 * i;
-    if (gm >= P.M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const long long gn = n0 + tx + 16 * j;
-      if (gn >= P.N) continue;
-      double* c = P.C + gm * P.ldc + gn;
-      *c = (P.beta == 0.0) ? acc[i][j] : fma(P.beta, *c, acc[i][j]);
-    }
-  }
-}
-
-
-// Register-blocked FP64 GEMM: CTA tile BM x BN, k-step 16, each of the 256
-// threads owns a TM x TN block of C; the next k-tile is prefetched into
-// registers while the current one is consumed from shared memory (double
-// buffered).  Same problem/segment tables and summation order per element as
-// gemm_grouped_f64: segments in table order, k ascending within a segment.
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256, 2) gemm_tiled_f64(const DGemmProblem* __restrict__ probs, int nprob,
-                                                      const DGemmSeg* __restrict__ segs) {
-  constexpr int BK = 8;
-  constexpr int NTX = BN / TN;  // threads along n
-  static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
-  constexpr int LA = BM * BK / 256, LB = BN * BK / 256;  // elements loaded per thread
-  __shared__ double As[2][BK][BM + 2];
-  __shared__ double Bs[2][BK][BN + 2];
-  const long long tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile_begin <= tile) lo = mid;
-    else hi = mid - 1;
-  }
-  const DGemmProblem P = probs[lo];
-  const long long t = tile - P.tile_begin;
-  const long long m0 = (t / P.tiles_n) * BM, n0 = (t % P.tiles_n) * BN;
-  const int tid = threadIdx.x, tx = tid % NTX, ty = tid / NTX;
-  double acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0;
-  for (long long sgi = P.seg_begin; sgi < P.seg_end; ++sgi) {
-    const DGemmSeg S = segs[sgi];
-    double ra[LA], rb[LB];
-    // the segment's alpha is folded into its B operand as it is loaded
-    auto load = [&](long long k0) {
-#pragma unroll
-      for (int u = 0; u < LA; ++u) {
-        const int e = tid + u * 256;
-        int mm, kk;
-        if (S.tA) { mm = e % BM; kk = e / BM; } else { kk = e % BK; mm = e / BK; }
-        const long long gm = m0 + mm, gk = k0 + kk;
-        ra[u] = (gm < P.M && gk < S.K) ? (S.tA ? S.A[gk * S.lda + gm] : S.A[gm * S.lda + gk]) : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int e = tid + u * 256;
-        int nn, kk;
-        if (S.tB) { kk = e % BK; nn = e / BK; } else { nn = e % BN; kk = e / BN; }
-        const long long gn = n0 + nn, gk = k0 + kk;
-        rb[u] = (gn < P.N && gk < S.K) ? S.alpha * (S.tB ? S.B[gn * S.ldb + gk] : S.B[gk * S.ldb + gn]) : 0.0;
-      }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-      for (int u = 0; u < LA; ++u) {
-        const int e = tid + u * 256;
-        int mm, kk;
-        if (S.tA) { mm = e % BM; kk = e / BM; } else { kk = e % BK; mm = e / BK; }
-        As[buf][kk][mm] = ra[u];
-      }
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int e = tid + u * 256;
-        int nn, kk;
-        if (S.tB) { kk = e % BK; nn = e / BK; } else { nn = e % BN; kk = e / BN; }
-        Bs[buf][kk][nn] = rb[u];
-      }
-    };
-    __syncthreads();  // previous segment finished reading the buffers
-    load(0);
-    store(0);
-    __syncthreads();
-    int buf = 0;
-    for (long long k0 = 0; k0 < S.K; k0 += BK) {
-      const bool more = k0 + BK < S.K;
-      if (more) load(k0 + BK);
-#pragma unroll
-      for (int kk = 0; kk < BK; ++kk) {
-        double a[TM], b[TN];
-#pragma unroll
-        for (int i = 0; i < TM; ++i) a[i] = As[buf][kk][ty + (BM / TM) * i];
-#pragma unroll
-        for (int j = 0; j < TN; ++j) b[j] = Bs[buf][kk][tx + NTX * j];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-      }
-      if (more) store(buf ^ 1);
-      __syncthreads();
-      buf ^= 1;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const long long gm = m0 + ty + (BM / TM) * i;
-    if (gm >= P.M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const long long gn = n0 + tx + NTX * j;
-      if (gn >= P.N) continue;
-      double* c = P.C + gm * P.ldc + gn;
-      *c = (P.beta == 0.0) ? acc[i][j] : fma(P.beta, *c, acc[i][j]);
-    }
-  }
-}
 
 // Skinny grouped GEMM (M <= SKINNY_M, B given as N x K): one warp per output
 // column n of a problem computes C[m][n] for every row m as dot products over
@@ -842,239 +646,6 @@ __global__ void __launch_bounds__(256) dom1_reverse(const D1Target* __restrict__
   T.R[(long long)q * n + b] += acc;
 }
 
-// Row-panel FP64 GEMM for problems with few rows and long rows of B (the all-external product Y = U W: a
-// few dozen gathered CI rows against the np x np operator): C (M x N) = beta C + sum over the segments of
-// alpha A B, A M x K and B K x N row major, M <= MT.  A block of 256 threads owns 128 columns of one problem
-// (tile_begin counts these column blocks).  B streams through shared memory in PANEL_KS-deep k slices by
-// 16-byte cp.async copies, PANEL_STG slices in flight (B is read from HBM exactly once, and enough bytes
-// are in flight to cover its latency); A's slices come the same way from L2.  Warp w computes rows
-// (w / 2) * MT/4 ... of the columns (w % 2) * 64 + 2 lane, +1: per pair of k a thread reads two 16-byte
-// B pairs and MT/4 16-byte A pairs (the same address across the warp) for MT FMAs.  Operands must start
-// on 16 bytes with even leading dimensions (checked when the step is lowered).  A segment's alpha scales
-// its B values as they are read.  Sums: segments in table order, k ascending.
-constexpr int PANEL_T = 256;
-constexpr int PANEL_COLS = 128;
-constexpr int PANEL_KS = 16;
-constexpr int PANEL_STG = 4;
-
-
-template <int MT>
-__global__ void __launch_bounds__(PANEL_T, 2) gemm_panel_f64(const DGemmProblem* __restrict__ probs, int nprob,
-                                                             const DGemmSeg* __restrict__ segs) {
-  constexpr int R = MT / 4;  // rows per warp
-  static_assert(MT % 8 == 0, "MT multiple of 8");
-  extern __shared__ __align__(16) double panel_smem[];
-  double* Ws = panel_smem;                                   // [PANEL_STG][PANEL_KS][PANEL_COLS]
-  double* As = panel_smem + PANEL_STG * PANEL_KS * PANEL_COLS;  // [PANEL_STG][MT][PANEL_KS]
-  const long long tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile_begin <= tile) lo = mid;
-    else hi = mid - 1;
-  }
-  const DGemmProblem P = probs[lo];
-  const long long n0 = (tile - P.tile_begin) * PANEL_COLS;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r0 = (warp >> 1) * R;
-  const int col = (warp & 1) * 64 + 2 * lane;  // this thread's two columns n0 + col, + 1
-  double acc[R][2];
-#pragma unroll
-  for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0.0;
-  for (long long sgi = P.seg_begin; sgi < P.seg_end; ++sgi) {
-    const DGemmSeg S = segs[sgi];
-    const long long K = S.K;
-    const long long nsl = (K + PANEL_KS - 1) / PANEL_KS;
-    const bool scaled = S.alpha != 1.0;
-    // one k slice of B (PANEL_KS x 128) and A (MT x PANEL_KS) into stage st, zero past the edges
-    auto issue = [&](long long sl, int st) {
-      const long long k0 = sl * PANEL_KS;
-      double* w = Ws + (size_t)st * PANEL_KS * PANEL_COLS;
-#pragma unroll
-      for (int u = 0; u < (PANEL_KS * PANEL_COLS / 2) / PANEL_T; ++u) {
-        const int e = tid + u * PANEL_T;               // 16-byte chunk
-        const int kk = e / (PANEL_COLS / 2), cc = 2 * (e % (PANEL_COLS / 2));
-        const long long gk = k0 + kk, gn = n0 + cc;
-        const int bytes = (gk < K && gn < P.N) ? (gn + 1 < P.N ? 16 : 8) : 0;
-        cp_async16(w + kk * PANEL_COLS + cc, bytes ? (const void*)(S.B + gk * S.ldb + gn) : (const void*)S.B, bytes);
-      }
-      double* a = As + (size_t)st * MT * PANEL_KS;
-      for (int e = tid; e < MT * PANEL_KS / 2; e += PANEL_T) {
-        const int m = e / (PANEL_KS / 2), kk = 2 * (e % (PANEL_KS / 2));
-        const long long gk = k0 + kk;
-        const int bytes = (m < P.M && gk < K) ? (gk + 1 < K ? 16 : 8) : 0;
-        cp_async16(a + m * PANEL_KS + kk, bytes ? (const void*)(S.A + m * S.lda + gk) : (const void*)S.A, bytes);
-      }
-    };
-    __syncthreads();  // the previous segment's stages have been read
-#pragma unroll
-    for (int st = 0; st < PANEL_STG - 1; ++st) {
-      if (st < nsl) issue(st, st);
-      cp_async_commit();
-    }
-    for (long long sl = 0; sl < nsl; ++sl) {
-      cp_async_wait<PANEL_STG - 2>();  // this thread's copies of slice sl have landed
-      __syncthreads();                 // everyone's have, and slice sl - 1 has been read
-      if (sl + PANEL_STG - 1 < nsl) issue(sl + PANEL_STG - 1, (int)((sl + PANEL_STG - 1) % PANEL_STG));
-      cp_async_commit();
-      const int st = (int)(sl % PANEL_STG);
-      const double* w = Ws + (size_t)st * PANEL_KS * PANEL_COLS + col;
-      const double* a = As + (size_t)st * MT * PANEL_KS + r0 * PANEL_KS;
-#pragma unroll
-      for (int kp = 0; kp < PANEL_KS / 2; ++kp) {
-        double2 w0 = *reinterpret_cast<const double2*>(w + (2 * kp) * PANEL_COLS);
-        double2 w1 = *reinterpret_cast<const double2*>(w + (2 * kp + 1) * PANEL_COLS);
-        if (scaled) {  // the segment's alpha on B, as gemm_tiled_f64 applies it
-          w0.x *= S.alpha, w0.y *= S.alpha, w1.x *= S.alpha, w1.y *= S.alpha;
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const double2 x = *reinterpret_cast<const double2*>(a + r * PANEL_KS + 2 * kp);
-          acc[r][0] = fma(x.y, w1.x, fma(x.x, w0.x, acc[r][0]));
-          acc[r][1] = fma(x.y, w1.y, fma(x.x, w0.y, acc[r][1]));
-        }
-      }
-    }
-    cp_async_wait<0>();
-  }
-  const long long n = n0 + col;
-  if (n >= P.N) return;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const long long m = r0 + r;
-    if (m >= P.M) break;
-    double* c = P.C + m * P.ldc + n;
-    c[0] = (P.beta == 0.0) ? acc[r][0] : fma(P.beta, c[0], acc[r][0]);
-    if (n + 1 < P.N) c[1] = (P.beta == 0.0) ? acc[r][1] : fma(P.beta, c[1], acc[r][1]);
-  }
-}
-template <int MT>
-constexpr size_t panel_smem_bytes() {
-  return sizeof(double) * (size_t)PANEL_STG * PANEL_KS * (PANEL_COLS + MT);
-}
-
-// Tiled FP64 GEMM with the operands staged by cp.async (the problem / segment tables and tile numbering
-// of gemm_tiled_f64<64, 128>): 64 x 128 tiles, 16-deep k slices, CP_STG slices in flight, 256 threads with
-// 4 x 8 outputs each (rows ty + 16 i, columns tx + 16 j).  A is M x K row major (tA = 0); B is K x N
-// (TB = 0, staged [k][n]) or N x K (TB = 1, staged [n][k] with its 16-byte chunks XOR-swizzled by the row
-// so that the column reads of a warp spread over the banks).  A segment's alpha scales its B values as
-// they are read, as in gemm_tiled_f64; segments in table order, k ascending.  Operands must start on
-// 16 bytes with even leading dimensions (checked when the step is lowered).
-constexpr int CP_BM = 64, CP_BN = 128, CP_BK = 16, CP_STG = 4;
-template <int TB>
-constexpr size_t cp_smem_bytes() {
-  return sizeof(double) * (size_t)CP_STG * (CP_BM * CP_BK + CP_BK * CP_BN);
-}
-template <int TB>
-__global__ void __launch_bounds__(256, 2) gemm_cp_f64(const DGemmProblem* __restrict__ probs, int nprob,
-                                                      const DGemmSeg* __restrict__ segs) {
-  extern __shared__ __align__(16) double cp_smem[];
-  double* As = cp_smem;                                  // [CP_STG][CP_BM][CP_BK]
-  double* Bs = cp_smem + CP_STG * CP_BM * CP_BK;         // [CP_STG][CP_BK][CP_BN] or [CP_STG][CP_BN][CP_BK]
-  const long long tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile_begin <= tile) lo = mid;
-    else hi = mid - 1;
-  }
-  const DGemmProblem P = probs[lo];
-  const long long t = tile - P.tile_begin;
-  const long long m0 = (t / P.tiles_n) * CP_BM, n0 = (t % P.tiles_n) * CP_BN;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  double acc[4][8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-  for (long long sgi = P.seg_begin; sgi < P.seg_end; ++sgi) {
-    const DGemmSeg S = segs[sgi];
-    const long long K = S.K;
-    const long long nsl = (K + CP_BK - 1) / CP_BK;
-    const double al = S.alpha;
-    auto issue = [&](long long sl, int st) {
-      const long long k0 = sl * CP_BK;
-      double* a = As + (size_t)st * CP_BM * CP_BK;
-      double* b = Bs + (size_t)st * CP_BK * CP_BN;
-      // A: 64 rows x 8 chunks = 512 chunks, 2 per thread
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int e = tid + u * 256;
-        const int m = e >> 3, kc = 2 * (e & 7);
-        const long long gm = m0 + m, gk = k0 + kc;
-        const int bytes = (gm < P.M && gk < K) ? (gk + 1 < K ? 16 : 8) : 0;
-        cp_async16(a + m * CP_BK + kc, bytes ? (const void*)(S.A + gm * S.lda + gk) : (const void*)S.A, bytes);
-      }
-      // B: 16 x 128 doubles = 1024 chunks, 4 per thread
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int e = tid + u * 256;
-        if (TB == 0) {
-          const int kk = e >> 6, nc = 2 * (e & 63);
-          const long long gk = k0 + kk, gn = n0 + nc;
-          const int bytes = (gk < K && gn < P.N) ? (gn + 1 < P.N ? 16 : 8) : 0;
-          cp_async16(b + kk * CP_BN + nc, bytes ? (const void*)(S.B + gk * S.ldb + gn) : (const void*)S.B, bytes);
-        } else {
-          const int nn = e >> 3, c = e & 7;  // row nn of B (a column of op(B)), chunk c of its 16 k
-          const long long gn = n0 + nn, gk = k0 + 2 * c;
-          const int bytes = (gn < P.N && gk < K) ? (gk + 1 < K ? 16 : 8) : 0;
-          cp_async16(b + nn * CP_BK + 2 * (c ^ (nn & 7)), bytes ? (const void*)(S.B + gn * S.ldb + gk) : (const void*)S.B,
-                     bytes);
-        }
-      }
-    };
-    __syncthreads();  // the previous segment's stages have been read
-#pragma unroll
-    for (int st = 0; st < CP_STG - 1; ++st) {
-      if (st < nsl) issue(st, st);
-      cp_async_commit();
-    }
-    for (long long sl = 0; sl < nsl; ++sl) {
-      cp_async_wait<CP_STG - 2>();
-      __syncthreads();
-      if (sl + CP_STG - 1 < nsl) issue(sl + CP_STG - 1, (int)((sl + CP_STG - 1) % CP_STG));
-      cp_async_commit();
-      const int st = (int)(sl % CP_STG);
-      const double* a = As + (size_t)st * CP_BM * CP_BK;
-      const double* b = Bs + (size_t)st * CP_BK * CP_BN;
-#pragma unroll
-      for (int kp = 0; kp < CP_BK / 2; ++kp) {
-        double2 x[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const double2*>(a + (ty + 16 * i) * CP_BK + 2 * kp);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          double b0, b1;
-          if (TB == 0) {
-            b0 = al * b[(2 * kp) * CP_BN + tx + 16 * j];
-            b1 = al * b[(2 * kp + 1) * CP_BN + tx + 16 * j];
-          } else {
-            const int nn = tx + 16 * j;
-            const double2 v = *reinterpret_cast<const double2*>(b + nn * CP_BK + 2 * (kp ^ (nn & 7)));
-            b0 = al * v.x;
-            b1 = al * v.y;
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[i][j] = fma(x[i].y, b1, fma(x[i].x, b0, acc[i][j]));
-        }
-      }
-    }
-    cp_async_wait<0>();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long gm = m0 + ty + 16 * i;
-    if (gm >= P.M) continue;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const long long gn = n0 + tx + 16 * j;
-      if (gn >= P.N) continue;
-      double* c = P.C + gm * P.ldc + gn;
-      *c = (P.beta == 0.0) ? acc[i][j] : fma(P.beta, *c, acc[i][j]);
-    }
-  }
-}
-
 // Segmented AXPY: target chunk t (at most AXPY_CHUNK elements) gets
 //   dst[i] += sum_s coef_s * scale_s * src_s[base + i].
 // One block per chunk; warp w takes the sources w, w + 8, ... in table order,
@@ -1568,11 +1139,8 @@ struct DevStep {
   int kind = 0;
   std::string name;
   // GEMM
-  DGemmProblem* probs = nullptr;
   DGemmSeg* segs = nullptr;
-  int nprob = 0;
-  long long ntiles = 0;
-  int cfg = 0;  // 0: 64x128 tiles, 1: 128x64 tiles
+  tci_dmma::Tables mma;  // FP64 form: every problem but the skinny ones
   // the same problems tiled for the tensor-core kernel (mixed-precision form)
   DGemmProblem* probs_tc = nullptr;
   DGemmSeg* segs_tc = nullptr;
@@ -1593,21 +1161,11 @@ struct DevStep {
   long long tma_rows = 0;  // kinds 4, 6, 7: rows of the gathered coefficients / of the exchange bank
   long long tma_aux2 = 0;  // kind 7: offset of the exchange bank in BUF_JK
   // FP64 form: problems with at most SKINNY_M rows and B given as N x K run on the skinny kernel
-  // FP64 problems on the cp.async-staged tiled kernel, by orientation of B
-  DGemmProblem* cp_probs[2] = {};
-  int cp_nprob[2] = {};
-  long long cp_ntiles[2] = {};
-  // FP64 problems of few rows on the row-panel kernel, by row class (M <= 16, 24, ..., 64)
-  DGemmProblem* panel_probs[7] = {};
-  int panel_nprob[7] = {};
-  long long panel_ntiles[7] = {};
   DGemmProblem* skinny_probs = nullptr;
   int skinny_nprob = 0;
   long long skinny_nwarps = 0;
-  DGemmProblem* probs_f = nullptr;  // its FP64 part (same-head one-electron-like segments)
+  tci_dmma::Tables mma_f;  // its FP64 part (same-head one-electron-like segments)
   DGemmSeg* segs_f = nullptr;
-  long long ntiles_f = 0;
-  int nprob_f = 0;
   bool tc_ok = false;  // worth the tensor cores: enough work and tiles mostly full
   // local decks: the two-external step on the heads' domains and common columns (gemm_com_f64)
   DComProblem* com_probs = nullptr;
@@ -2568,6 +2126,17 @@ struct tci_ctx {
     return it != loc_pos.end() && *it < off + len;
   }
 
+  tci_dmma::Tables mma_tables(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& sg) {
+    const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
+    tci_dmma::Tables d;
+    for (int c = 0; c < tci_dmma::CLASSES; ++c) {
+      d.probs[c] = upload(t.probs[c], owned, stream);
+      d.nprob[c] = (int)t.probs[c].size();
+      d.ntiles[c] = t.ntiles[c];
+    }
+    return d;
+  }
+
   DevStep lower(const Step& s) {
     DevStep d;
     d.kind = s.kind;
@@ -2575,21 +2144,10 @@ struct tci_ctx {
     if (s.kind == STEP_GEMM) {
       std::vector<DGemmProblem> pr;
       std::vector<DGemmSeg> sg;
-      long long tiles = 0;
-      // tile shape: wide in n when the problems are short in m (e.g. few CI blocks times an operator)
-      double sm = 0, sn = 0;
       for (auto& g : s.gp) {
-        sm += (double)g.M;
-        sn += (double)g.N;
-      }
-      d.cfg = (sm <= sn) ? 0 : 1;
-      const i64 BMh = d.cfg == 0 ? 64 : 128, BNh = d.cfg == 0 ? 128 : 64;
-      for (auto& g : s.gp) {
-        const i64 tm = (g.M + BMh - 1) / BMh, tn = (g.N + BNh - 1) / BNh;
         if (g.M <= 0 || g.N <= 0) continue;
         check_range(g.c, g.offC, (g.M - 1) * g.ldc + g.N);
-        pr.push_back(DGemmProblem{ptr(g.c, g.offC), g.ldc, g.M, g.N, tn, tiles, g.beta, g.seg_begin, g.seg_end, 0});
-        tiles += tm * tn;
+        pr.push_back(DGemmProblem{ptr(g.c, g.offC), g.ldc, g.M, g.N, 0, 0, g.beta, g.seg_begin, g.seg_end, 0});
       }
       for (auto& g : s.gs) sg.push_back(DGemmSeg{ptr(g.a, g.offA), ptr(g.b, g.offB), g.lda, g.ldb, g.K, g.tA, g.tB, g.alpha});
       // full operand extents: A is M x K (K x M if transposed), B is K x N (N x K)
@@ -2607,73 +2165,26 @@ struct tci_ctx {
       }
       d.segs = upload(sg, owned, stream);
       {
-        // FP64 form: skinny problems (one-row products) to the warp-per-column kernel, the rest tiled
-        std::vector<DGemmProblem> reg, sk, pan[7], cpp[2];
-        long long rt = 0, wk = 0, pt[7] = {0, 0, 0, 0, 0, 0, 0}, ct[2] = {0, 0};
+        // FP64 form: skinny problems (one-row products) to the warp-per-column kernel, the rest to the matrix
+        // instruction
+        std::vector<DGemmProblem> sk, reg;
+        long long wk = 0;
         for (const auto& g : pr) {
           bool skinny = g.M <= SKINNY_M && s.name != "all-external";
           for (long long q = g.seg_begin; skinny && q < g.seg_end; ++q) skinny = sg[(size_t)q].tA == 0 && sg[(size_t)q].tB == 1;
-          // few rows against long rows of B (the all-external product: a few dozen CI rows x the operator;
-          // the reverse three-external product: the pair-matrix rows x the (iq|bs) banks) on the row-panel
-          // kernel when the operands allow 16-byte copies
-          bool panel = g.M <= 64 && g.N >= 1024 && !skinny;
-          for (long long q = g.seg_begin; panel && q < g.seg_end; ++q) {
-            const DGemmSeg& x = sg[(size_t)q];
-            panel = x.tA == 0 && x.tB == 0 && ((x.lda | x.ldb) & 1) == 0 &&
-                    ((reinterpret_cast<uintptr_t>(x.A) | reinterpret_cast<uintptr_t>(x.B)) & 15) == 0;
-          }
-          if (panel) {
-            const int c = (int)((g.M + 7) / 8) - 1;  // MT = 8 (c + 1), classes 16 ... 64
-            const int cls = std::max(1, c) - 1;       // 0: MT 16, 1: 24, ..., 6: 64
-            DGemmProblem x = g;
-            x.tile_begin = pt[cls];
-            pt[cls] += (g.N + PANEL_COLS - 1) / PANEL_COLS;
-            pan[cls].push_back(x);
-          } else if (skinny) {
+          if (skinny) {
             DGemmProblem x = g;
             x.tile_begin = wk;  // first warp (one per output column); a block of 8 warps stays in one problem
             wk += (g.N + 7) / 8 * 8;
             sk.push_back(x);
           } else {
-            // the cp.async-staged tiled kernel where the operands allow 16-byte copies (A not transposed,
-            // one orientation of B per problem), else the register-staged one
-            bool cpk = true;
-            int tb = -1;
-            for (long long q = g.seg_begin; cpk && q < g.seg_end; ++q) {
-              const DGemmSeg& x = sg[(size_t)q];
-              cpk = x.tA == 0 && (tb < 0 || tb == x.tB) && ((x.lda | x.ldb) & 1) == 0 &&
-                    ((reinterpret_cast<uintptr_t>(x.A) | reinterpret_cast<uintptr_t>(x.B)) & 15) == 0;
-              tb = x.tB;
-            }
-            DGemmProblem x = g;
-            if (cpk && tb >= 0) {
-              x.tiles_n = (g.N + CP_BN - 1) / CP_BN;
-              x.tile_begin = ct[tb];
-              ct[tb] += ((g.M + CP_BM - 1) / CP_BM) * x.tiles_n;
-              cpp[tb].push_back(x);
-            } else {
-              x.tile_begin = rt;
-              rt += ((g.M + BMh - 1) / BMh) * x.tiles_n;
-              reg.push_back(x);
-            }
+            reg.push_back(g);
           }
         }
-        d.probs = upload(reg, owned, stream);
-        d.nprob = (int)reg.size();
-        d.ntiles = rt;
-        for (int b = 0; b < 2; ++b) {
-          d.cp_probs[b] = upload(cpp[b], owned, stream);
-          d.cp_nprob[b] = (int)cpp[b].size();
-          d.cp_ntiles[b] = ct[b];
-        }
+        d.mma = mma_tables(reg, sg);
         d.skinny_probs = upload(sk, owned, stream);
         d.skinny_nprob = (int)sk.size();
         d.skinny_nwarps = wk;
-        for (int c = 0; c < 7; ++c) {
-          d.panel_probs[c] = upload(pan[c], owned, stream);
-          d.panel_nprob[c] = (int)pan[c].size();
-          d.panel_ntiles[c] = pt[c];
-        }
       }
       if (s.name != "all-external" && !pr.empty()) {
         // Mixed form.  Segments whose operand is a same-head one-electron-like operator (BUF_F: h, J_ii,
@@ -2699,8 +2210,7 @@ struct tci_ctx {
         }
         std::vector<DGemmProblem> pf, pt;
         std::vector<DGemmSeg> sf, st;
-        d.ntiles_f = tci_dev::tile_problems(f64, tci_dev::gemm_f64_tile_m(d.cfg), tci_dev::gemm_f64_tile_n(d.cfg), false,
-                                            pf, sf);
+        tci_dev::tile_problems(f64, 64, 64, false, pf, sf);
         // 128 x 64 tiles; a problem short in M is computed transposed
         d.ntiles_tc = tci_dev::tile_problems(tcp, tci_gtc_host::tile_m(), tci_gtc_host::tile_n(), true, pt, st);
         double flops = 0, useful = 0, issued = 0;
@@ -2712,9 +2222,8 @@ struct tci_ctx {
           useful += (double)g.M * (double)g.N * k;
           issued += (double)((g.M + TM - 1) / TM * TM) * (double)((g.N + TN - 1) / TN * TN) * k;
         }
-        d.probs_f = upload(pf, owned, stream);
+        d.mma_f = mma_tables(pf, sf);
         d.segs_f = upload(sf, owned, stream);
-        d.nprob_f = (int)pf.size();
         d.probs_tc = upload(pt, owned, stream);
         d.segs_tc = upload(st, owned, stream);
         d.nprob_tc = (int)pt.size();
@@ -2909,33 +2418,6 @@ struct tci_ctx {
            (s.tma_kind == 4 && tma_ss_ready) || (s.tma_kind == 5 && tma_1x_ready) || (s.tma_kind == 6 && tma_dv_ready) ||
            (s.tma_kind == 7 && tma_dvr_ready);
   }
-  template <int TB>
-  void launch_cp(const DevStep& s) {
-    if (s.cp_ntiles[TB] <= 0) return;
-    constexpr size_t smem = cp_smem_bytes<TB>();
-    static bool attr_set[64] = {};  // per device
-    int dev = 0;
-    TCI_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-      TCI_CUDA(cudaFuncSetAttribute(gemm_cp_f64<TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr_set[dev] = true;
-    }
-    gemm_cp_f64<TB><<<(unsigned)s.cp_ntiles[TB], 256, smem, stream>>>(s.cp_probs[TB], s.cp_nprob[TB], s.segs);
-  }
-  template <int MT>
-  void launch_panel(const DevStep& s, int c) {
-    if (s.panel_ntiles[c] <= 0) return;
-    constexpr size_t smem = panel_smem_bytes<MT>();
-    static bool attr_set[64] = {};  // per device
-    int dev = 0;
-    TCI_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-      TCI_CUDA(cudaFuncSetAttribute(gemm_panel_f64<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr_set[dev] = true;
-    }
-    gemm_panel_f64<MT><<<(unsigned)s.panel_ntiles[c], PANEL_T, smem, stream>>>(s.panel_probs[c], s.panel_nprob[c],
-                                                                               s.segs);
-  }
   // the mixed form runs this GEMM step on the tensor cores
   bool uses_tc(const DevStep& s) const {
     return precision == 1 && s.probs_tc && (tc_mode == 1 || (tc_mode == 0 && s.tc_ok));
@@ -2969,17 +2451,14 @@ struct tci_ctx {
       }
       if (s.kind == STEP_GEMM && uses_tc(s)) {
         const bool f_in_tma = f_on_tc && s.tma_kind == 1 && s.tma_probs && tma_ok(s);
-        k += (s.skinny_nwarps > 0 ? 1 : 0) + ((s.ntiles_f > 0 && !f_in_tma) ? 1 : 0) +
+        k += (s.skinny_nwarps > 0 ? 1 : 0) + (f_in_tma ? 0 : s.mma_f.launches()) +
              ((s.tma_probs && tma_ok(s)) ? 2 : (s.ntiles_tc > 0 ? 1 : 0));
         continue;
       }
       if (s.kind == STEP_GEMM && s.skinny_nwarps > 0) k += 1;
-      if (s.kind == STEP_GEMM) {
-        for (int c = 0; c < 7; ++c) k += s.panel_ntiles[c] > 0 ? 1 : 0;
-        for (int b = 0; b < 2; ++b) k += s.cp_ntiles[b] > 0 ? 1 : 0;
-      }
+      if (s.kind == STEP_GEMM) k += s.mma.launches();
       if (s.zc_ntg > 0) k += 1;
-      if ((s.kind == STEP_GEMM && s.ntiles > 0) || ((s.kind == STEP_AXPY || s.kind == STEP_DOT) && s.ntg > 0) ||
+      if (((s.kind == STEP_AXPY || s.kind == STEP_DOT) && s.ntg > 0) ||
           ((s.kind == STEP_UNPACK || s.kind == STEP_PACK) && plan.nD > 0))
         k += 1;
     }
@@ -3384,7 +2863,7 @@ struct tci_ctx {
             s.tma_probs && tma_ok(s)) {
           const i64 n = plan.n;
           if (s.tma_kind == 1) {
-            if (!f_on_tc) TCI_CUDA(tci_dev::launch_gemm_f64(s.cfg, s.probs_f, s.nprob_f, s.segs_f, s.ntiles_f, stream));
+            if (!f_on_tc) TCI_CUDA(tci_dmma::launch(s.mma_f, s.segs_f, stream));
             TCI_CUDA(tci_gtma_host::split(buf[BUF_D], plan.nD * n, n, n, d_hi, d_lo, stream));
             TCI_CUDA(tci_gtma_host::launch(tma_dd, s.tma_probs, s.tma_nprob, s.tma_segs, s.tma_ntiles, (int)tc_kblock,
                                            tc_status, stream));
@@ -3417,26 +2896,14 @@ struct tci_ctx {
           break;
         }
         if (uses_tc(s)) {
-          TCI_CUDA(tci_dev::launch_gemm_f64(s.cfg, s.probs_f, s.nprob_f, s.segs_f, s.ntiles_f, stream));
+          TCI_CUDA(tci_dmma::launch(s.mma_f, s.segs_f, stream));
           TCI_CUDA(tci_gtc_host::launch(s.probs_tc, s.nprob_tc, s.segs_tc, s.ntiles_tc, tc_status, (int)tc_kblock, stream));
           break;
         }
         if (s.skinny_nwarps > 0)
           gemm_skinny_f64<<<(unsigned)((s.skinny_nwarps + 7) / 8), 256, 0, stream>>>(s.skinny_probs, s.skinny_nprob,
                                                                                   s.segs, s.skinny_nwarps);
-        launch_panel<16>(s, 0);
-        launch_panel<24>(s, 1);
-        launch_panel<32>(s, 2);
-        launch_panel<40>(s, 3);
-        launch_panel<48>(s, 4);
-        launch_panel<56>(s, 5);
-        launch_panel<64>(s, 6);
-        launch_cp<0>(s);
-        launch_cp<1>(s);
-        if (s.ntiles > 0) {
-          if (s.cfg == 0) gemm_tiled_f64<64, 128, 4, 8><<<(unsigned)s.ntiles, 256, 0, stream>>>(s.probs, s.nprob, s.segs);
-          else gemm_tiled_f64<128, 64, 8, 4><<<(unsigned)s.ntiles, 256, 0, stream>>>(s.probs, s.nprob, s.segs);
-        }
+        TCI_CUDA(tci_dmma::launch(s.mma, s.segs, stream));
         break;
       case STEP_AXPY:
         if (s.ntg > 0) {
@@ -3472,32 +2939,7 @@ struct tci_ctx {
   }
 };
 
-namespace tci_dev {
-cudaError_t launch_gemm_cp_f64(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles,
-                               cudaStream_t st) {
-  if (ntiles <= 0 || nprob <= 0) return cudaSuccess;
-  constexpr size_t smem = cp_smem_bytes<0>();
-  static bool attr_set[64] = {};  // per device
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    e = cudaFuncSetAttribute(gemm_cp_f64<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
-  }
-  gemm_cp_f64<0><<<(unsigned)ntiles, 256, smem, st>>>(probs, nprob, segs);
-  return cudaGetLastError();
-}
 
-cudaError_t launch_gemm_f64(int cfg, const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles,
-                            cudaStream_t st) {
-  if (ntiles <= 0 || nprob <= 0) return cudaSuccess;
-  if (cfg == 0) gemm_tiled_f64<64, 128, 4, 8><<<(unsigned)ntiles, 256, 0, st>>>(probs, nprob, segs);
-  else gemm_tiled_f64<128, 64, 8, 4><<<(unsigned)ntiles, 256, 0, st>>>(probs, nprob, segs);
-  return cudaGetLastError();
-}
-}  // namespace tci_dev
 
 extern "C" {
 

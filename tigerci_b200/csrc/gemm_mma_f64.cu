@@ -8,15 +8,16 @@
 // pipe, not shared memory or issue slots, sets the rate (the scalar tiled kernels it replaced ran at 10-24 TFLOP/s).
 // Four warps own a 64 x 128 tile, each 64 x 32 of it in 128 accumulator registers, two blocks per SM so that one's
 // copies and barriers run under the other's products; four 16-deep slices in flight by cp.async. Measured on a B200:
-// 592 problems of 256 x 256 x (40 x 256) 30 TFLOP/s, 576 of 173 x 173 x (40 x 173) 20 (6 % of the blocks padding,
-// uneven column shares). Against the scalar kernels: two-external step at 24 pairs x 173 virtuals 102 -> 40 ms, all-
-// external at 240 virtuals 6.8 -> 5.1 ms. Tried and slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp
+// 592 problems of 256 x 256 x (40 x 256) 31 TFLOP/s, 576 of 173 x 173 x (40 x 173) 23 (6 % of the blocks padding,
+// uneven column shares; 20 with one body for all shapes and predicates for the missing blocks). Against the scalar
+// kernels: two-external step at 24 pairs x 173 virtuals 102 -> 35 ms, all-external at 240 virtuals 6.8 -> 5.1 ms. Tried and slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp
 // that only copies (registers spill at two blocks per SM), the copies dealt between the products (the loop outgrows
 // the instruction cache: 9-17).
 #include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <stdexcept>
+#include <type_traits>
 #include <utility>
 
 #include "../../include/tigerci_sigma.h"
@@ -245,30 +246,41 @@ __global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __rest
     produce(st == 0 ? STG - 1 : st - 1);
     const double* as = sm + st * Sh::STAGE;
     const double* bs = as + bo + (KB ? (mk >> (9 + (tq & 1))) & 1 : 0);
-    auto step = [&](int s4) {  // four k
-      const int fo = (f0 ^ ((s4 & 3) << 2)) + (s4 >> 2) * 16;
-      double a[MB];
+    // The warp's R x N blocks of the slice.  One body per shape: a matrix instruction whose predicate is off still
+    // takes its slot of the pipe.
+    auto body = [&](auto rr, auto nn) {
+      constexpr int R = decltype(rr)::value, N = decltype(nn)::value;
+      auto step = [&](int s4) {  // four k
+        const int fo = (f0 ^ ((s4 & 3) << 2)) + (s4 >> 2) * 16;
+        double a[R > 0 ? R : 1];
 #pragma unroll
-      for (int i = 0; i < MB; ++i) a[i] = as[i * 8 * BK + fo];
+        for (int i = 0; i < R; ++i) a[i] = as[i * 8 * BK + fo];
 #pragma unroll
-      for (int j = 0; j < NB; ++j) {
-        if (j >= nb) break;
-        double b = KB ? bs[s4 * 4 * Sh::B::PITCH + j * 8] : bs[j * 8 * BK + fo];
-        if (mk & 256) b *= al;
+        for (int j = 0; j < N; ++j) {
+          double b = KB ? bs[s4 * 4 * Sh::B::PITCH + j * 8] : bs[j * 8 * BK + fo];
+          if (mk & 256) b *= al;
 #pragma unroll
-        for (int i = 0; i < MB - 1; ++i) mma884(acc[i][j][0], acc[i][j][1], a[i], b);
-        if (mb == MB) mma884(acc[MB - 1][j][0], acc[MB - 1][j][1], a[MB - 1], b);
+          for (int i = 0; i < R; ++i) mma884(acc[i][j][0], acc[i][j][1], a[i], b);
+        }
+      };
+      if constexpr (WK == 1) {
+#pragma unroll
+        for (int s4 = 0; s4 < BK / 4; ++s4)
+          if (4 * s4 < kc) step(s4);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (8 * role + 4 * q < kc) step(2 * role + q);
       }
     };
-    if constexpr (WK == 1) {
-#pragma unroll
-      for (int s4 = 0; s4 < BK / 4; ++s4)
-        if (4 * s4 < kc) step(s4);
-    } else {
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-        if (8 * role + 4 * q < kc) step(2 * role + q);
-    }
+    auto bodies = [&](auto rr) {
+      if (nb == 4) body(rr, std::integral_constant<int, 4>());
+      else if (nb == 3) body(rr, std::integral_constant<int, 3>());
+      else if (nb == 2) body(rr, std::integral_constant<int, 2>());
+      else if (nb == 1) body(rr, std::integral_constant<int, 1>());
+    };
+    if (mb == MB) bodies(std::integral_constant<int, MB>());
+    else bodies(std::integral_constant<int, MB - 1>());
     st = st == STG - 1 ? 0 : st + 1;
   }
   cp_wait<0>();

@@ -19,13 +19,17 @@
 //   T_hk (Jc n_h x n_h) = [L^J_h]_J (Jc n_h x n_h) D_hk
 //   R_hk (n_h x n_h)   += 1/2 sum_J T_hkJ L^J_h       (Jc K-segments of n_h)
 //
-// on the FP64 SIMT kernel or, in the mixed form, on the TMA-fed tcgen05 3xTF32
+// on the FP64 matrix-instruction kernel or, in the mixed form, on the TMA-fed tcgen05 3xTF32
 // kernel: there L^J_h, D_hk and T_hk live as TF32-high / FP32-low rows (pitch a
 // multiple of 32, zero past each domain), the first GEMM writes T_hk directly
 // in that split form and the second accumulates R_hk in FP64.
-// The chunk size and the FP64 tile shape of the second GEMM come from a small
+// The chunk size (mixed form: and the first GEMM's tile width) comes from a small
 // autotuner that times each candidate once at set-up.  One application
 // (unpack, chunks, pack) is captured as one CUDA graph.
+//
+// In FP64 the packed integrals X = Lpk Lpk^T over all externals replace the
+// Cholesky vectors where they pay (local_integral.cu): n_h^4 / 2 products per
+// block on the domain instead of 4 nchol n_h^3, bound by one streaming of X.
 //
 // In the mixed form a second, dense form competes with it: the packed
 // integral form of the non-local all-external term (W+ over the pairs (aa)
@@ -59,6 +63,7 @@
 #include "gemm_mma_f64.h"
 #include "gemm_tables.h"
 #include "gemm_tma.h"
+#include "local_integral.h"
 #include "host/capi_internal.h"
 
 using namespace tci;
@@ -301,7 +306,9 @@ struct tci_local {
   tci_gtma_host::TmaMaps map1, map1n, map2;  // T = Lc D (128- or 64-wide tiles) ; R += 1/2 T Lc
   TmaLaunch m1, m2, m1r, m2r;
   // dense padded integral form (mixed precision): W+ / W- over all externals as FP32 tiles
-  int form = 0;              // form in use: 0 Cholesky, 1 dense
+  int form = 0;              // form in use: 0 Cholesky, 1 dense, 2 integrals on the domains (FP64)
+  double* X = nullptr;       // form 2: (ab|cd), npv x npv
+  tci_lint::Device lint;
   bool dense_ready = false;  // the dense operators are built
   int64_t np_d = 0, nm_d = 0, nsing_d = 0, ntrip_d = 0;
   float *w32p = nullptr, *w32m = nullptr, *u2p = nullptr, *u2m = nullptr;
@@ -485,6 +492,59 @@ struct tci_local {
     dense_ready = true;
   }
 
+  // Integral form (FP64): the kernel's tables, host side.
+  void plan_integral(const std::vector<long long>& dom, tci_lint::Plan& P) const {
+    std::vector<int> di, dp;
+    for (const auto& H : heads) {
+      dp.push_back((int)di.size());
+      for (long long a = 0; a < H.n; ++a) di.push_back((int)dom[(size_t)(H.dom_off + a)]);
+    }
+    std::vector<tci_lint::Block> bl;
+    for (const auto& B : blocks)
+      bl.push_back(tci_lint::Block{B.ab ? B.off_ab + B.k * (B.n * (B.n - 1) / 2) : -1, B.aa ? B.off_aa + B.k * B.n : -1, B.p,
+                                   (int)B.n, dp[(size_t)B.head], (int)B.head, 0});
+    tci_lint::make_plan((int)nvirt, (int)heads.size(), di, std::move(bl), (int)tci_dev::device_sms(), P);
+  }
+  // Its set-up from the virtual-virtual Cholesky rows lpk: X by row panels of its lower triangle on the FP64 GEMM,
+  // mirrored, and the tables.
+  void build_integral(const double* lpk, const tci_lint::Plan& P) {
+    X = alloc((size_t)(npv * npv));
+    std::vector<DGemmProblem> pr;
+    std::vector<DGemmSeg> sg;
+    constexpr long long PANEL = 2048;
+    for (long long r = 0; r < npv; r += PANEL) {
+      const long long m = std::min<long long>(PANEL, npv - r);
+      pr.push_back(DGemmProblem{X + r * npv, npv, m, r + m, 0, 0, 0.0, (long long)sg.size(), (long long)sg.size() + 1, 0});
+      sg.push_back(DGemmSeg{lpk + r * nchol, lpk, nchol, nchol, nchol, 0, 1, 1.0});
+    }
+    GemmLaunch g;
+    const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
+    for (int c = 0; c < tci_dmma::CLASSES; ++c) {
+      g.t.probs[c] = upload(t.probs[c]);
+      g.t.nprob[c] = (int)t.probs[c].size();
+      g.t.ntiles[c] = t.ntiles[c];
+    }
+    g.segs = upload(sg);
+    launch_gemm(g);
+    LCUDA(tci_lint::mirror(X, npv, stream));
+    lint.blocks = upload(P.blocks);
+    lint.tasks = upload(P.tasks);
+    lint.jobs = upload(P.jobs);
+    lint.cblk = upload(P.cblk);
+    lint.jcol = upload(P.jcol);
+    lint.dom = upload(P.dom);
+    lint.pos = upload(P.pos);
+    lint.nblocks = (int)P.blocks.size();
+    lint.ntasks = (int)P.tasks.size();
+    lint.nv = P.nv;
+    lint.parts = P.parts;
+    const size_t cl = P.blocks.size() * (size_t)P.nv * (size_t)tci_lint::pitch(P.nv);
+    lint.C = alloc(cl);
+    LCUDA(cudaMemsetAsync(lint.C, 0, sizeof(double) * cl, stream));  // zero outside the domains, for good
+    if (P.parts > 1) lint.part = alloc((size_t)P.parts * (size_t)total);
+    LCUDA(cudaStreamSynchronize(stream));  // the host tables above go out of scope
+  }
+
   // Dense form, one application: Sb = [U+ W+ ; U- W-] gathered from and scattered to the local blocks.
   void record_dense() {
     const unsigned nb = (unsigned)blocks.size();
@@ -506,6 +566,11 @@ struct tci_local {
     const unsigned nb = (unsigned)blocks.size();
     if (form == 1) {
       record_dense();
+      return;
+    }
+    if (form == 2) {
+      LCUDA(cudaMemsetAsync(Sb, 0, sizeof(double) * (size_t)total, stream));
+      LCUDA(tci_lint::launch(lint, X, npv, Cb, Sb, total, stream));
       return;
     }
     if (precision == 1) {
@@ -560,10 +625,10 @@ struct tci_local {
     }
     capture();
   }
-  // Graph of the dense form.
-  void configure_dense() {
+  // Graph of the dense (1) or the integral (2) form.
+  void configure_form(int f) {
     release_graph();
-    form = 1;
+    form = f;
     capture();
   }
   // one application captured as the graph in use
@@ -633,8 +698,8 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
     const double budget = (options && n_options > 1 && options[1] > 0) ? (double)options[1] : 16e9;
     if (options && n_options > 2 && options[2] > 0) L->kblock = options[2];
     const bool tune = !(options && n_options > 3 && options[3] == 0);
-    const int64_t want_form = (options && n_options > 4) ? options[4] : 0;  // 0 faster, 1 Cholesky, 2 dense
-    if (want_form < 0 || want_form > 2) throw Error(TCI_ERR_ARG, "unknown all-external form");
+    const int64_t want_form = (options && n_options > 4) ? options[4] : 0;  // 0 faster, 1 Cholesky, 2 dense, 3 integral
+    if (want_form < 0 || want_form > 3) throw Error(TCI_ERR_ARG, "unknown all-external form");
     if (L->precision < 0 || L->precision > 1 || L->kblock % 32) throw Error(TCI_ERR_ARG, "bad precision or promotion block");
     // heads and blocks (host checks: every index below is bounds-checked here, not on the device)
     long long dtot = 0, lc_per_j = 0, t_per_j = 0, dom_total = 0, lrows = 0, drows = 0, nmax = 0;
@@ -713,7 +778,29 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       if (B.aa && B.p < 0.0) dense = false;
     if (want_form == 2 && !dense)
       throw Error(TCI_ERR_INPUT, "the dense all-external form needs the mixed precision and singlet-coupled aa blocks");
-    const bool chol_form = want_form != 2;
+    // FP64: the integrals on the domains where the device has room for X and it costs no more to set up than the
+    // Cholesky form's timed runs (X takes npv^2 nchol flops, three runs 3 x flops; at 150 pairs of 20-150 of 300
+    // externals the application goes 81 -> 11 ms), a caller's chunk budget below the default bounding X too
+    bool integral = L->precision == 0 && want_form != 1 && want_form != 2 && num_external <= tci_lint::MAX_NV;
+    for (const auto& B : L->blocks)
+      if (B.aa && B.p < 0.0) integral = false;
+    if (want_form == 3 && !integral)
+      throw Error(TCI_ERR_INPUT, "the integral all-external form needs FP64 and singlet-coupled aa blocks");
+    tci_lint::Plan iplan;
+    if (integral) {
+      const double xb = 8.0 * (double)L->npv * (double)L->npv;
+      const double cb = 8.0 * (double)L->blocks.size() * (double)num_external * (double)tci_lint::pitch(num_external);
+      const double need = xb + cb + 8.0 * (double)L->npv * (double)nchol + 80.0 * (double)total_len + 2e9;
+      size_t free_b = 0, total_b = 0;
+      LCUDA(cudaMemGetInfo(&free_b, &total_b));
+      const bool room = need < (want_form == 3 ? 1.0 : 0.6) * (double)free_b;
+      if (want_form == 3 && !room) throw Error(TCI_ERR_MEMORY, "not enough device memory for the integral all-external form");
+      integral = want_form == 3 || (room && (budget >= 16e9 || xb + cb <= budget) &&
+                                    3.0 * L->flops >= (double)L->npv * (double)L->npv * (double)nchol);
+      if (integral) L->plan_integral(dom, iplan);
+      if (want_form != 3 && 1.5 * iplan.flops > L->flops) integral = false;
+    }
+    const bool chol_form = want_form != 2 && !integral;
     if (dense) {
       // device bytes it needs at set-up (X, the split Cholesky rows, the W tiles, U and Y), with the
       // Cholesky form's buffers when both are timed, against what the device has free
@@ -746,6 +833,7 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       double* tmp = L->alloc(lvv.size());
       LCUDA(cudaMemcpyAsync(tmp, lvv.data(), lvv.size() * sizeof(double), cudaMemcpyHostToDevice, L->stream));
       if (dense) L->build_dense(tmp);
+      if (integral) L->build_integral(tmp, iplan);
       if (chol_form) {
         L->LT = L->alloc(lvv.size());
         dim3 grid((unsigned)((nchol + 31) / 32), (unsigned)((L->npv + 31) / 32));
@@ -813,8 +901,9 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       L->tuned_ms = best;
       if (pick != std::make_pair(L->jc, L->cfg2)) L->configure(pick.first, pick.second);
     }
+    if (integral) L->configure_form(2);
     if (L->dense_ready) {
-      L->configure_dense();
+      L->configure_form(1);
       L->time_once();
       L->dense_ms = L->time_once();
       L->check_status();

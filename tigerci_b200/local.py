@@ -20,9 +20,9 @@ import numpy as np
 from ._lib import check, lib, ptr
 
 PRECISIONS = {"fp64": 0, "tf32x3": 1}
-# all-external form: the faster of the two (timed at set-up), the pair-domain Cholesky form, or the dense
-# padded integral form (mixed precision only)
-FORMS = {"auto": 0, "cholesky": 1, "dense": 2}
+# all-external form: the faster one, the pair-domain Cholesky form, the dense padded integral form (mixed precision
+# only) or the integrals on the domains (FP64 only)
+FORMS = {"auto": 0, "cholesky": 1, "dense": 2, "integral": 3}
 
 
 def _bind():
@@ -69,7 +69,7 @@ class LocalAllExternal:
         check(self._L.tci_local_apply(self._h, C.c_void_p(c_ptr), C.c_void_p(s_ptr), self.n, C.c_void_p(stream or None)))
 
     def stats(self) -> dict:
-        """form: "cholesky" or "dense" (the one applied); tuned_ms / dense_ms: the set-up timings of the two forms
+        """form: "cholesky", "dense" or "integral" (the one applied); tuned_ms / dense_ms: the set-up timings of the two forms
         (0 where a form was not timed); flops: the Cholesky form's 4 nchol sum n^3, dense_flops: the dense form's
         2 np^2 per singlet-coupled and 2 nm^2 per triplet-coupled block; dense_w_bytes: its FP32 W tiles."""
         out = np.zeros(13)
@@ -77,7 +77,7 @@ class LocalAllExternal:
         keys = ["flops", "cholesky_bytes", "device_bytes", "chunk", "tile_cfg", "tuned_ms", "candidates", "last_ms",
                 "blocks", "form", "dense_ms", "dense_flops", "dense_w_bytes"]
         d = dict(zip(keys, out.tolist()))
-        d["form"] = "dense" if d["form"] == 1 else "cholesky"
+        d["form"] = ("cholesky", "dense", "integral")[int(d["form"])]
         return d
 
     def close(self):

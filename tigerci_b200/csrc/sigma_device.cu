@@ -36,6 +36,7 @@
 #include "gemm_tma.h"
 #include "host/capi_internal.h"
 #include "host/plan.h"
+#include "local_com.h"
 
 using namespace tci;
 
@@ -168,51 +169,10 @@ __global__ void __launch_bounds__(256) gemm_skinny_f64(const DGemmProblem* __res
     }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-// 8-byte form (gathers of single elements); src_bytes 0 fills the destination with zeros
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, int src_bytes) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
-}
-
-// Domain-restricted two-external products of a local deck (pair domains) over the common virtuals, as the
-// reference takes them (two_int_seg_com_lmo_res, three_and_four_seg_mod_2.f90:7137-8005, GEMMs at :7718-7751).
-// Source head mu's pair matrix is zero outside D_mu x D_mu and the target head lambda needs only
-// D_lambda x D_lambda, so a term reaches only the columns in both domains:
-//   R_lambda[a][b] += alpha sum_{c in D_mu} X[a][c] D_mu[c][b]      (a in D_lambda, b in D_lambda and D_mu)
-// m_lambda x |common| x m_mu per term instead of m_lambda x m_lambda x m_mu. The step works on compact squares:
-// per sigma build the pair matrices of the local heads are gathered into m x m squares (com_gather_sq), the
-// products accumulate into compact m x m accumulators (zeroed first) that are then added into the padded ones
-// (com_scatter_sq); the integral operands X[D_lambda][D_mu] are constant and compacted once at set-up when the
-// device has room (com_pack_a), else gathered from the n x n matrices. Each term carries its common columns as
-// positions in the source's and in the target's domain. A block owns 64 rows of one target and walks all its
-// (term, 32-column chunk, 16-deep k chunk) in table order, the operands copied by 8-byte cp.async
-// COM_STG - 1 chunks ahead of the FMAs (one barrier per chunk); at the end of each column chunk it adds alpha
-// times its 64 x 32 sums into the target's square. Every element is written by one block, its terms in table
-// order, and the barrier between two column chunks orders the read-modify-writes of different threads: the sum
-// stays in a fixed order.
-struct DComProblem {
-  double* C;         // the target's compact accumulator (m x m, row pitch `pitch`)
-  const int* dom;    // the target's domain (rows of the gathered integral operand)
-  int m, pitch;
-  long long tile_begin, seg_begin, seg_end;
-};
-struct DComSeg {
-  const double* A;   // the n x n integral operand (gathered when Ac is nullptr)
-  const double* Ac;  // A[D_target][D_source], row pitch pitch_a, or nullptr
-  const double* B;   // the source's compact pair matrix, row pitch pitch_b
-  const int* dom;    // the source's domain (the k range)
-  const int* cs;     // the common columns: positions in the source's domain ...
-  const int* ct;     // ... and in the target's
-  int m, ncol, pitch_a, pitch_b;
-  double alpha;
-};
+// The two-external products of a local deck run on local_com.cu over compact squares: per sigma build the pair
+// matrices of the local heads are gathered into m x m squares (com_gather_sq); the integral operands
+// X[D_lambda][D_mu] are constant and compacted once at set-up when the device has room (com_pack_a), else gathered
+// from the n x n matrices.
 // one compaction job: Ac[r][c] = A[rows[r]][cols[c]] (r < m, c < ms), row pitch `pitch`
 struct DComPack {
   const double* A;
@@ -242,147 +202,6 @@ __global__ void __launch_bounds__(256) com_gather_sq(const DComSq* __restrict__ 
     Q.sq[(long long)r * Q.pitch + c] = Q.pad[(long long)Q.dom[r] * ld + Q.dom[c]];
   }
 }
-__global__ void __launch_bounds__(256) com_scatter_sq(const DComSq* __restrict__ sq, long long ld) {
-  const DComSq Q = sq[blockIdx.x];
-  for (int e = threadIdx.x; e < Q.m * Q.m; e += blockDim.x) {
-    const int r = e / Q.m, c = e - r * Q.m;
-    Q.pad[(long long)Q.dom[r] * ld + Q.dom[c]] += Q.sq[(long long)r * Q.pitch + c];
-  }
-}
-constexpr int COM_R = 64, COM_C = 32, COM_K = 16, COM_THREADS = 128, COM_STG = 3;
-// position in a block's (segment, column chunk, k chunk) sequence
-struct ComCursor {
-  long long s;
-  int c, k;
-};
-__global__ void __launch_bounds__(COM_THREADS, 4) gemm_com_f64(const DComProblem* __restrict__ probs, int nprob,
-                                                              const DComSeg* __restrict__ segs, long long ld) {
-  __shared__ __align__(16) double As[COM_STG][COM_K][COM_R];
-  __shared__ __align__(16) double Bs[COM_STG][COM_K][COM_C];
-  const long long tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile_begin <= tile) lo = mid;
-    else hi = mid - 1;
-  }
-  const DComProblem P = probs[lo];
-  if (P.seg_begin >= P.seg_end) return;
-  const int r0 = (int)(tile - P.tile_begin) * COM_R;
-  // outputs: rows 8 ty .. 8 ty + 7, columns tx and tx + 16 of the chunk
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // copy slots: A rows ia + 8 q at k = ka; B rows kb + 4 q at column jb
-  const int ka = tid & 15, ia = tid >> 4, kb = tid >> 5, jb = tid & 31;
-  auto advance = [&](ComCursor& x, const DComSeg& S) {
-    x.k += COM_K;
-    if (x.k < S.m) return;
-    x.k = 0;
-    x.c += COM_C;
-    if (x.c < S.ncol) return;
-    x.c = 0;
-    ++x.s;
-  };
-  // the copies of one chunk into stage st (zeros past the domains, the rows or the common columns)
-  auto issue = [&](const ComCursor& x, const DComSeg& S, int st) {
-    const int k = x.k + ka;
-    if (S.Ac) {  // compacted: 16 consecutive k of a row across the 16 threads of a row group
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int r = r0 + ia + 8 * q;
-        const bool ok = r < P.m && k < S.m;
-        cp_async8(&As[st][ka][ia + 8 * q], ok ? (const void*)(S.Ac + (long long)r * S.pitch_a + k) : (const void*)S.Ac,
-                  ok ? 8 : 0);
-      }
-    } else {
-      const long long col = k < S.m ? (long long)S.dom[k] : -1;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int r = r0 + ia + 8 * q;
-        const bool ok = r < P.m && col >= 0;
-        cp_async8(&As[st][ka][ia + 8 * q], ok ? (const void*)(S.A + (long long)P.dom[r] * ld + col) : (const void*)S.A,
-                  ok ? 8 : 0);
-      }
-    }
-    const int bc = x.c + jb < S.ncol ? S.cs[x.c + jb] : -1;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int kk = x.k + kb + 4 * q;
-      const bool ok = kk < S.m && bc >= 0;
-      cp_async8(&Bs[st][kb + 4 * q][jb], ok ? (const void*)(S.B + (long long)kk * S.pitch_b + bc) : (const void*)S.B,
-                ok ? 8 : 0);
-    }
-  };
-  // producer cursor: COM_STG - 1 chunks ahead of the consumer
-  ComCursor pc{P.seg_begin, 0, 0};
-  DComSeg PS = segs[pc.s];
-  for (int st = 0; st < COM_STG - 1; ++st) {
-    if (pc.s < P.seg_end) {
-      issue(pc, PS, st);
-      advance(pc, PS);
-      if (pc.s < P.seg_end && pc.c == 0 && pc.k == 0) PS = segs[pc.s];
-    }
-    cp_async_commit();
-  }
-  ComCursor cc{P.seg_begin, 0, 0};
-  DComSeg S = segs[cc.s];
-  double acc[8][2];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0.0;
-  for (int it = 0;; ++it) {
-    const int st = it % COM_STG;
-    cp_async_wait<COM_STG - 2>();  // this thread's copies of the chunk have landed
-    __syncthreads();               // everyone's have, and the stage refilled below is no longer read
-#pragma unroll
-    for (int k = 0; k < COM_K; ++k) {
-      const double2* ap = reinterpret_cast<const double2*>(&As[st][k][8 * ty]);
-      double a[8];
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const double2 v = ap[h];
-        a[2 * h] = v.x;
-        a[2 * h + 1] = v.y;
-      }
-      const double b0 = Bs[st][k][tx], b1 = Bs[st][k][tx + 16];
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        acc[r][0] = fma(a[r], b0, acc[r][0]);
-        acc[r][1] = fma(a[r], b1, acc[r][1]);
-      }
-    }
-    // the copies COM_STG - 1 chunks ahead, after the FMAs so that their index loads overlap them
-    if (pc.s < P.seg_end) {
-      issue(pc, PS, (it + COM_STG - 1) % COM_STG);
-      advance(pc, PS);
-      if (pc.s < P.seg_end && pc.c == 0 && pc.k == 0) PS = segs[pc.s];
-    }
-    cp_async_commit();
-    const ComCursor prev = cc;
-    advance(cc, S);
-    if (cc.s != prev.s || cc.c != prev.c) {  // this column chunk is complete: add it into the target's square
-      int ct[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int j = prev.c + tx + 16 * c;
-        ct[c] = j < S.ncol ? S.ct[j] : -1;
-      }
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int i = r0 + 8 * ty + r;
-        if (i >= P.m) continue;
-        double* row = P.C + (long long)i * P.pitch;
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-          if (ct[c] >= 0) row[ct[c]] += S.alpha * acc[r][c];
-      }
-#pragma unroll
-      for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0.0;
-      if (cc.s >= P.seg_end) break;
-      if (cc.s != prev.s) S = segs[cc.s];
-    }
-  }
-  cp_async_wait<0>();
-}
-
 // Domain-restricted three-external products of a local deck (pair domains), on the padded pair matrices and
 // the (iq|bs) banks V_i[b][q n + s] (the reference's local three-external gathers, iabc_sig_cho_big_res,
 // three_and_four_seg_mod_1.f90:1099-1376). The pair matrices of an N-2 head lambda are zero outside
@@ -1167,19 +986,12 @@ struct DevStep {
   tci_dmma::Tables mma_f;  // its FP64 part (same-head one-electron-like segments)
   DGemmSeg* segs_f = nullptr;
   bool tc_ok = false;  // worth the tensor cores: enough work and tiles mostly full
-  // local decks: the two-external step on the heads' domains and common columns (gemm_com_f64)
-  DComProblem* com_probs = nullptr;
-  DComSeg* com_segs = nullptr;
-  int com_nprob = 0;
-  long long com_ntiles = 0;
+  // local decks: the two-external step on the heads' domains and common columns (local_com.cu)
+  tci_com::Tables com;
   DComPack* com_pack = nullptr;  // compaction of its constant operands, run once after the set-up steps
   long long com_njobs = 0;
-  DComSq* com_gather = nullptr;   // pair matrices -> compact squares
+  DComSq* com_gather = nullptr;  // pair matrices -> compact squares
   long long com_ngather = 0;
-  DComSq* com_scatter = nullptr;  // compact accumulators -> padded ones
-  long long com_nscatter = 0;
-  double* com_rsq = nullptr;      // the compact accumulators (zeroed per build)
-  long long com_rsq_len = 0;
   bool com_step = false;
   // local decks: the zero-external rows of N-2 and N-1 heads on the common positions (axpy_common)
   ZcTarget* zc_tg = nullptr;
@@ -1666,9 +1478,8 @@ struct tci_ctx {
       owned.push_back(*p);
       bytes_held += (double)std::max<i64>(1, len) * sizeof(double);
     };
-    double *dsq = nullptr, *rsq = nullptr;
+    double* dsq = nullptr;
     dev_alloc(&dsq, sq_len);
-    dev_alloc(&rsq, sq_len);
     const int* ddom = upload(ls.dh_dom, owned, stream);
     const int* dcs = upload(cpos_s, owned, stream);
     const int* dct = upload(cpos_t, owned, stream);
@@ -1702,8 +1513,8 @@ struct tci_ctx {
         jobs.push_back(DComPack{std::get<0>(kv.first), abuf + kv.second, ddom + ls.dh_off[(size_t)ht],
                                 ddom + ls.dh_off[(size_t)hs], (int)mh(ht), (int)mh(hs), (int)pitch_of(mh(hs))});
       }
-    // the squares: gathered sources (those some term reads), zeroed and scattered targets
-    std::vector<DComSq> gsq, ssq;
+    // the gathered squares: the sources that some term reads
+    std::vector<DComSq> gsq;
     for (i64 dk = 0; dk < plan.nD; ++dk) {
       if (sq_off[(size_t)dk] < 0) continue;
       const i64 h = dk2h[(size_t)dk];
@@ -1711,36 +1522,52 @@ struct tci_ctx {
                (int)pitch_of(mh(h))};
       if (src_used[(size_t)dk]) gsq.push_back(q);
     }
-    std::vector<DComProblem> pr;
-    std::vector<DComSeg> sg;
-    long long tiles = 0;
+    // tasks: even row tiles of each target, the longest first; jobs: each term's common columns, COLS at a time
+    std::vector<tci_com::Job> cj;
+    struct HostTask {
+      double work;
+      tci_com::Task t;
+    };
+    std::vector<HostTask> ct[tci_com::CLASSES];
     for (const auto& p : probs) {
-      ssq.push_back(DComSq{buf[BUF_R] + p.dk * n2, rsq + sq_off[(size_t)p.dk], ddom + ls.dh_off[(size_t)p.head],
-                           (int)p.m, (int)pitch_of(p.m)});
-      DComProblem P{rsq + sq_off[(size_t)p.dk], ddom + ls.dh_off[(size_t)p.head], (int)p.m, (int)pitch_of(p.m),
-                    tiles, (long long)sg.size(), 0};
+      const int cls = tci_com::task_class((int)p.m);
+      if (cls < 0) throw Error(TCI_ERR_INPUT, "pair domain too large for the two-external step");
+      const int job0 = (int)cj.size();
+      double work = 0;
       for (const auto& x : p.segs) {
         const i64 ms = mh(x.hs);
         const double* ac = abuf ? abuf + apos.at(std::make_tuple(x.A, p.head, x.hs)) : nullptr;
-        sg.push_back(DComSeg{x.A, ac, dsq + sq_off[(size_t)x.dks], ddom + ls.dh_off[(size_t)x.hs], dcs + x.col_off,
-                             dct + x.col_off, (int)ms, (int)x.ncol, (int)pitch_of(ms), (int)pitch_of(ms), x.alpha});
+        const i64 parts = (x.ncol + tci_com::COLS - 1) / tci_com::COLS;
+        for (i64 q = 0; q < parts; ++q) {
+          const i64 f = x.ncol * q / parts, e = x.ncol * (q + 1) / parts;
+          cj.push_back(tci_com::Job{ac ? ac : x.A, dsq + sq_off[(size_t)x.dks], ddom + ls.dh_off[(size_t)x.hs],
+                                    dcs + x.col_off + f, dct + x.col_off + f, (int)ms, (int)(e - f), (int)pitch_of(ms),
+                                    (int)pitch_of(ms), x.alpha, ac ? 1 : 0, 0});
+          work += (double)((ms + 15) / 16) * (double)(8 + (e - f));
+        }
       }
-      P.seg_end = (long long)sg.size();
-      tiles += (p.m + COM_R - 1) / COM_R;
-      pr.push_back(P);
+      const int rows = tci_com::class_rows(cls), nt = ((int)p.m + rows - 1) / rows;
+      for (int t = 0; t < nt; ++t) {
+        const int f = (int)(p.m * t / nt), e = (int)(p.m * (t + 1) / nt);
+        ct[cls].push_back(HostTask{work, tci_com::Task{buf[BUF_R] + p.dk * n2, ddom + ls.dh_off[(size_t)p.head], (int)p.m, f,
+                                                       e - f, job0, (int)cj.size(), 0}});
+      }
     }
-    d.com_probs = upload(pr, owned, stream);
-    d.com_segs = upload(sg, owned, stream);
-    d.com_nprob = (int)pr.size();
-    d.com_ntiles = tiles;
+    for (int c = 0; c < tci_com::CLASSES; ++c) {
+      std::stable_sort(ct[c].begin(), ct[c].end(), [](const HostTask& x, const HostTask& y) { return x.work > y.work; });
+      std::vector<tci_com::Task> v;
+      for (const auto& x : ct[c]) {
+        v.push_back(x.t);
+        d.com.mmax[c] = std::max(d.com.mmax[c], x.t.m);
+      }
+      d.com.tasks[c] = upload(v, owned, stream);
+      d.com.ntasks[c] = (int)v.size();
+    }
+    d.com.jobs = upload(cj, owned, stream);
     d.com_pack = upload(jobs, owned, stream);
     d.com_njobs = (long long)jobs.size();
     d.com_gather = upload(gsq, owned, stream);
     d.com_ngather = (long long)gsq.size();
-    d.com_scatter = upload(ssq, owned, stream);
-    d.com_nscatter = (long long)ssq.size();
-    d.com_rsq = rsq;
-    d.com_rsq_len = sq_len;
     d.com_step = true;
     return d;
   }
@@ -2427,7 +2254,7 @@ struct tci_ctx {
     long long k = 0;
     for (const auto& s : sigma) {
       if (s.com_step) {
-        k += (s.com_ngather > 0 ? 1 : 0) + (s.com_ntiles > 0 ? 1 : 0) + (s.com_nscatter > 0 ? 1 : 0);
+        k += (s.com_ngather > 0 ? 1 : 0) + s.com.launches();
         continue;
       }
       if (s.d3_skip) continue;
@@ -2842,13 +2669,7 @@ struct tci_ctx {
         if (s.com_step) {  // local deck: the two-external step on the domains
           if (s.com_ngather > 0)
             com_gather_sq<<<(unsigned)s.com_ngather, 256, 0, stream>>>(s.com_gather, plan.n);
-          if (s.com_ntiles > 0) {
-            TCI_CUDA(cudaMemsetAsync(s.com_rsq, 0, (size_t)s.com_rsq_len * sizeof(double), stream));
-            gemm_com_f64<<<(unsigned)s.com_ntiles, COM_THREADS, 0, stream>>>(s.com_probs, s.com_nprob, s.com_segs,
-                                                                           plan.n);
-          }
-          if (s.com_nscatter > 0)
-            com_scatter_sq<<<(unsigned)s.com_nscatter, 256, 0, stream>>>(s.com_scatter, plan.n);
+          TCI_CUDA(tci_com::launch(s.com, plan.n, stream));
           break;
         }
         if (tc_allext && s.name == "all-external") {

@@ -42,9 +42,13 @@
 // rounds the same in either order, so the result does not depend on which
 // CTA finishes first.
 //
-// Warp roles (448 threads): warps 0-3 and 10-13 epilogue (two per TMEM lane
-// quadrant), warps 4-7 low parts of the W tile, warp 8 producer (bulk copy +
-// TMA), warp 9 TMEM allocator + MMA issuer.  Every mbarrier wait is bounded; on timeout
+// Warp roles (832 threads): warps 0-15 epilogue (four per TMEM lane quadrant), warps 16-23 low parts of the W
+// tile (two sets of four, alternate stages), warp 24 producer (bulk copy + TMA), warp 25 TMEM allocator + MMA
+// issuer.  The pace was set by single threads' instruction latencies: the issuer's divisions, abort-flag reads and
+// descriptor arithmetic took 420 of the 1290 cycles a k-step lasted at 240 virtuals, its waits and MMAs the rest,
+// and the epilogue's eight warps then held the accumulators back (350 cycles a step).  With counters instead of
+// divisions and sixteen epilogue warps a step takes 1010 cycles: 1.98 -> 1.75 ms per sigma build there.  A fifth
+// stage or another L2 lead changes nothing.  Every mbarrier wait is bounded; on timeout
 // the kernel records an error code, drains and returns (no trap).
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -76,8 +80,9 @@ constexpr int B_BYTES = 2 * W_BYTES;        // W tile (its own high part) + low 
 constexpr int A_BYTES = 2 * BN * BK * 4;    // 16 KB: interleaved U rows (room for the largest group)
 constexpr int STAGE_BYTES = B_BYTES + A_BYTES;
 constexpr int TMEM_COLS = 2 * MMA_N;        // two accumulator buffers
-constexpr int NTHREADS = 448;
-constexpr int EPI_WARPS = 8;  // warps 0-3 and 10-13: two per TMEM lane quadrant, each half of the panel
+constexpr int NTHREADS = 832;
+constexpr int EPI_WARPS = 16;  // warps 0-15: four per TMEM lane quadrant, each a quarter of the panel
+constexpr int CONV_WARP = EPI_WARPS, PROD_WARP = CONV_WARP + 8, MMA_WARP = PROD_WARP + 1;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 9) {  // TMEM: 2 accumulator buffers of MMA_N fp32 columns
+  if (warp == MMA_WARP) {  // TMEM: 2 accumulator buffers of MMA_N fp32 columns
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -234,31 +239,41 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   };
   auto aborted = [&]() { return *(volatile int*)abort_flag != 0; };
 
-  if (warp == 8) {
+  if (warp == PROD_WARP) {
     // ---------------- producer: W tile by bulk copy (L2 lead), U rows by TMA ----------------
     if (lane == 0) {
       int step = 0, last = -1;  // k-steps issued so far in this CTA; the last one
-      for (long long pos = begin; pos < end && !aborted();) {
+      int s = 0;
+      uint32_t ph = 1;          // parity of the stage's last refill: passes at once in the first round
+      bool ok = true;
+      for (long long pos = begin; pos < end && ok;) {
         const Segment g = segment_at(p0, p1, pos, end);
-        const float* wt = (g.prod ? p1.W : p0.W) + (long long)g.panel * (g.prod ? p1.nk : p0.nk) * TILE_FLOATS;
+        const float* wt = (g.prod ? p1.W : p0.W) + ((long long)g.panel * (g.prod ? p1.nk : p0.nk) + g.k0) * TILE_FLOATS;
         const CUtensorMap* u_map = g.prod ? &u_map1 : &u_map0;
-        const int bn = g.prod ? p1.bn : p0.bn;
+        const int bn = g.prod ? p1.bn : p0.bn, urow = g.group * 2 * bn, n = g.k1 - g.k0;
         const uint32_t bytes = (uint32_t)(W_BYTES + 2 * bn * BK * 4);
-        for (int k = g.k0; k < g.k0 + PREFETCH && k < g.k1; ++k) bulk_prefetch_l2(wt + (long long)k * TILE_FLOATS, W_BYTES);
-        for (int k = g.k0; k < g.k1 && !aborted(); ++k, ++step) {
-          const int s = step % STAGES;
-          if (step >= STAGES && !mbar_wait(&empty[s], ((step / STAGES) - 1) & 1)) {
+        for (int k = 0; k < PREFETCH && k < n; ++k) bulk_prefetch_l2(wt + (long long)k * TILE_FLOATS, W_BYTES);
+        int x = g.k0 * BK;
+        for (int k = 0; k < n; ++k, ++step, x += BK, wt += TILE_FLOATS) {
+          if (!mbar_wait(&empty[s], ph)) {
             fail(ST_TIMEOUT_EMPTY);
+            ok = false;
             break;
           }
-          if (k + PREFETCH < g.k1) bulk_prefetch_l2(wt + (long long)(k + PREFETCH) * TILE_FLOATS, W_BYTES);
           uint8_t* st = base + s * STAGE_BYTES;
           mbar_expect_tx(&full[s], bytes);
-          bulk_load(st, wt + (long long)k * TILE_FLOATS, W_BYTES, &full[s]);
-          tma_load_2d(st + B_BYTES, u_map, &full[s], k * BK, g.group * 2 * bn);
+          bulk_load(st, wt, W_BYTES, &full[s]);
+          tma_load_2d(st + B_BYTES, u_map, &full[s], x, urow);
           last = step;
+          if (k + PREFETCH < n) bulk_prefetch_l2(wt + (long long)PREFETCH * TILE_FLOATS, W_BYTES);
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1;
+            ok = !aborted();
+            if (!ok) break;
+          }
         }
-        pos += g.k1 - g.k0;
+        pos += n;
       }
       if (aborted()) {
         // the copies of the last STAGES issued k-steps may still be landing: wait (bounded) for them
@@ -267,11 +282,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           mbar_wait(&full[st % STAGES], (st / STAGES) & 1);
       }
     }
-  } else if (warp >= 4 && warp < 8) {
+  } else if (warp >= CONV_WARP && warp < PROD_WARP) {
     // ---------------- low parts of the W tile: rows BM.. of the B operand ----------------
-    const int cw = warp - 4;
+    // (STAGES even: a set always meets the same stages, so no phase passes unseen)
+    static_assert(STAGES % 2 == 0, "stages per converter set");
+    const int cw = warp & 3;
     const long long nsteps = end - begin;
-    for (long long step = 0; step < nsteps && !aborted(); ++step) {
+    for (long long step = (warp - CONV_WARP) >> 2; step < nsteps && !aborted(); step += 2) {
       const int s = (int)(step % STAGES);
       if (!mbar_wait(&full[s], (uint32_t)((step / STAGES) & 1))) {
         fail(ST_TIMEOUT_FULL);
@@ -295,38 +312,45 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&conv[s]);
     }
-  } else if (warp == 9) {
+  } else if (warp == MMA_WARP) {
     // ---------------- MMA issuer: promotion blocks of KB_PER_BLOCK steps, never across segments ----------------
     if (lane == 0) {
+      // One thread's instruction latencies are the pace here: no division, abort flag read once per block,
+      // descriptors by additions.
       const uint32_t idesc = idesc_tf32(2 * BN, MMA_N);
-      int step = 0, blk = 0;
-      for (long long pos = begin; pos < end && !aborted();) {
+      const uint64_t da0 = smem_desc_sw128(base + B_BYTES), db0 = smem_desc_sw128(base);
+      int s = 0, blk = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (long long pos = begin; pos < end && ok;) {
         const Segment g = segment_at(p0, p1, pos, end);
-        for (int k = g.k0; k < g.k1 && !aborted(); ++k, ++step) {
-          const int kin = k - g.k0;
-          const bool first = (kin % KB_PER_BLOCK) == 0;
-          const int buf = blk & 1;
-          if (first && blk >= 2 && !mbar_wait(&dempty[buf], ((blk / 2) - 1) & 1)) {
+        for (int left = g.k1 - g.k0; left > 0 && ok; left -= KB_PER_BLOCK, ++blk) {
+          const int buf = blk & 1, n = left < KB_PER_BLOCK ? left : KB_PER_BLOCK;
+          if (blk >= 2 && !mbar_wait(&dempty[buf], ((blk >> 1) - 1) & 1)) {
             fail(ST_TIMEOUT_DE);
+            ok = false;
             break;
           }
-          const int s = step % STAGES;
-          if (!mbar_wait(&conv[s], (step / STAGES) & 1)) {
-            fail(ST_TIMEOUT_CONV);
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          uint8_t* st = base + s * STAGE_BYTES;
           const uint32_t d = tmem + (uint32_t)(buf * MMA_N);
+          for (int i = 0; i < n; ++i) {
+            if (!mbar_wait(&conv[s], ph)) {
+              fail(ST_TIMEOUT_CONV);
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint64_t da = da0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (STAGE_BYTES >> 4));
 #pragma unroll
-          for (int kk = 0; kk < BK / 8; ++kk)  // 8 tf32 = 32 bytes of every row per MMA
-            mma_tf32(d, smem_desc_sw128(st + B_BYTES + kk * 32), smem_desc_sw128(st + kk * 32), idesc,
-                     (first && kk == 0) ? 0u : 1u);
-          mma_commit(&empty[s]);
-          if ((kin % KB_PER_BLOCK) == KB_PER_BLOCK - 1 || k == g.k1 - 1) {
-            mma_commit(&dfull[buf]);
-            ++blk;
+            for (int kk = 0; kk < BK / 8; ++kk)  // 8 tf32 = 32 bytes of every row per MMA
+              mma_tf32(d, da + 2 * kk, db + 2 * kk, idesc, (i == 0 && kk == 0) ? 0u : 1u);
+            mma_commit(&empty[s]);
+            if (++s == STAGES) {
+              s = 0;
+              ph ^= 1;
+            }
           }
+          if (ok) mma_commit(&dfull[buf]);
+          if (aborted()) ok = false;
         }
         pos += g.k1 - g.k0;
       }
@@ -336,15 +360,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         mbar_wait(mma_done, 0);
       }
     }
-  } else if (warp < 4 || warp >= 10) {
+  } else {
     // ---------------- epilogue: lane pairs joined, FP32 block sums -> FP64 registers -> Y ----------------
     // TMEM lane quadrant q = warp mod 4: lane l is U row 32 q + l = CI block 16 q + l / 2, high (even)
-    // or low (odd) part; warps 0-3 take panel columns 0-63, warps 10-13 columns 64-127.  Per 8-column
+    // or low (odd) part; warps 4 c .. 4 c + 3 take panel columns 32 c .. 32 c + 31.  Per 8-column
     // chunk the even lane keeps columns 0-3 and the odd lane 4-7 after the pair exchange.
-    const int q = warp & 3, half = warp >= 10 ? 1 : 0;
+    const int q = warp & 3, part = warp >> 2;
     const int odd = lane & 1;
     const int jl = 16 * q + (lane >> 1);  // CI block within the group
-    constexpr int COLS = BM / 2;          // panel columns per warp
+    constexpr int COLS = 4 * BM / EPI_WARPS;  // panel columns per warp
     int blk = 0;
     for (long long pos = begin; pos < end && !aborted();) {
       const Segment g = segment_at(p0, p1, pos, end);
@@ -362,7 +386,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
         if (active) {
           asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t dq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * MMA_N + half * COLS);
+          const uint32_t dq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * MMA_N + part * COLS);
 #pragma unroll
           for (int c0 = 0; c0 < COLS / 8; c0 += 2) {  // two 8-column chunks per wait
             uint32_t vh[2][8], vl[2][8];
@@ -394,7 +418,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         for (int c = 0; c < COLS / 8; ++c)
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const int r = g.panel * BM + half * COLS + c * 8 + (odd ? 4 : 0) + t;
+            const int r = g.panel * BM + part * COLS + c * 8 + (odd ? 4 : 0) + t;
             // one or two CTAs add into the zeroed output (see the header)
             if (r < P.np) atomicAdd(&P.Y[(long long)j * P.ldy + r], acc[c * 4 + t]);
           }
@@ -405,7 +429,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  if (warp == MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
 // FP64 W (np x np) -> FP32 tiles (W at init): tile (panel, k) holds rows panel BM .. +BM-1, columns

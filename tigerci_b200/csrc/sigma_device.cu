@@ -853,59 +853,77 @@ cudaError_t dev_malloc(T** p, size_t bytes, cudaStream_t st) {
 }
 inline cudaError_t dev_free(void* p, cudaStream_t st) { return p ? cudaFreeAsync(p, st) : cudaSuccess; }
 
-// partial[k * RBLK + b] = sum over block b's chunk of A[k][i] * x[i].  Four rows per pass share the loads
-// of x (each row's products are still summed in the order of the one-row loop).
+// partial[k * gridDim.x + b] = sum over chunk b of A[k][i] * x[i]: block (b, g) takes the rows 4 g .. 4 g + 3, which
+// share the loads of x. Bound by HBM (the rows once; x comes from L2 for the other row groups): a thread's products
+// are summed in ascending i, four iterations' loads in flight (with one block walking all rows and one iteration's
+// loads at a time, 27 rows of 1,971,105 took 129 us against 68 at the copy bandwidth).
 __global__ void __launch_bounds__(RB) multi_dot_partial(const double* __restrict__ A, long long lda, int m,
                                                         const double* __restrict__ x, long long n,
                                                         double* __restrict__ partial) {
   __shared__ double red[4][RB / 32];
   const long long chunk = (n + gridDim.x - 1) / gridDim.x;
   const long long i0 = (long long)blockIdx.x * chunk, i1 = min(n, i0 + chunk);
-  for (int k0 = 0; k0 < m; k0 += 4) {
-    const int nk = min(4, m - k0);
-    const double* a0 = A + (long long)k0 * lda;
-    const double* a1 = nk > 1 ? a0 + lda : a0;
-    const double* a2 = nk > 2 ? a0 + 2 * lda : a0;
-    const double* a3 = nk > 3 ? a0 + 3 * lda : a0;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (long long i = i0 + threadIdx.x; i < i1; i += RB) {
-      const double xi = x[i];
-      acc[0] = fma(a0[i], xi, acc[0]);
-      acc[1] = fma(a1[i], xi, acc[1]);
-      acc[2] = fma(a2[i], xi, acc[2]);
-      acc[3] = fma(a3[i], xi, acc[3]);
-    }
+  const int k0 = 4 * blockIdx.y, nk = min(4, m - k0);
+  const double* a[4];
+  a[0] = A + (long long)k0 * lda;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+  for (int q = 1; q < 4; ++q) a[q] = q < nk ? a[0] + q * lda : a[0];
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  long long i = i0 + threadIdx.x;
+  for (; i + 3 * RB < i1; i += 4 * RB) {
+    double xv[4], v[4][4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-      if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = acc[q];
-    }
-    __syncthreads();
-    if (threadIdx.x < nk) {
-      double t = 0.0;
-      for (int w = 0; w < RB / 32; ++w) t += red[threadIdx.x][w];
-      partial[(long long)(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
-    }
-    __syncthreads();
+    for (int u = 0; u < 4; ++u) xv[u] = x[i + u * RB];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[q][u] = q < nk ? a[q][i + u * RB] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = fma(v[q][u], xv[u], acc[q]);
+  }
+  for (; i < i1; i += RB) {
+    const double xi = x[i];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[q] = fma(a[q][i], xi, acc[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = acc[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < nk) {
+    double t = 0.0;
+    for (int w = 0; w < RB / 32; ++w) t += red[threadIdx.x][w];
+    partial[(long long)(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
   }
 }
 
-__global__ void multi_dot_final(const double* __restrict__ partial, int m, int nblk, double* __restrict__ out) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
+// out[k] = sign x the sum of row k's RBLK partials in ascending order (the solver's projections and, negated, the
+// coefficients of a classical Gram-Schmidt pass): one block per row brings them to shared memory at once, one
+// thread adds (a chain of loads from L2 took 25 us).
+__global__ void __launch_bounds__(128) multi_dot_final(const double* __restrict__ partial, double sign,
+                                                       double* __restrict__ out) {
+  __shared__ double p[RBLK];
+  for (int b = threadIdx.x; b < RBLK; b += blockDim.x) p[b] = partial[(long long)blockIdx.x * RBLK + b];
+  __syncthreads();
+  if (threadIdx.x) return;
   double t = 0.0;
-  for (int b = 0; b < nblk; ++b) t += partial[(long long)k * nblk + b];
-  out[k] = t;
+#pragma unroll 16
+  for (int b = 0; b < RBLK; ++b) t += p[b];
+  out[blockIdx.x] = sign * t;
 }
 
-// out[k] = -(sum of the partials of k): the coefficients of one classical Gram-Schmidt pass
-__global__ void multi_dot_final_neg(const double* __restrict__ partial, int m, int nblk, double* __restrict__ out) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
+// tci_dots: out[k] = the sum of row k's nblk partials, a warp per row (fixed order: lanes, then a shuffle tree)
+__global__ void __launch_bounds__(32) dots_final(const double* __restrict__ partial, int nblk, double* __restrict__ out) {
   double t = 0.0;
-  for (int b = 0; b < nblk; ++b) t += partial[(long long)k * nblk + b];
-  out[k] = -t;
+  for (int b = threadIdx.x; b < nblk; b += 32) t += partial[(long long)blockIdx.x * nblk + b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // out[i] = beta*out[i] + sum_k ca[k] A[k][i] + sum_k cb[k] B[k][i]
@@ -1076,6 +1094,7 @@ struct tci_ctx {
   double last_sigma_ms = 0;
   long long sigma_count = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev_last = nullptr;  // the last asynchronous device work of an entry point (never recorded in a capture)
   bool profiling = false;
   bool use_graph = true;                // replay the sigma steps as one CUDA graph
   int64_t precision = 0;                // 0 plain FP64; 1 all-external on tcgen05 (3xTF32, FP64 promotion)
@@ -1161,6 +1180,7 @@ struct tci_ctx {
     if (stream) cudaStreamSynchronize(stream);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    if (ev_last) cudaEventDestroy(ev_last);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -2175,8 +2195,8 @@ struct tci_ctx {
 
   // out[0..m) = A[k] . x  (host result), deterministic
   void multi_dot(const double* A, i64 lda, int m, const double* x, i64 n, double* host_out) {
-    multi_dot_partial<<<RBLK, RB, 0, stream>>>(A, lda, m, x, n, dots);
-    multi_dot_final<<<(m + 127) / 128, 128, 0, stream>>>(dots, m, RBLK, dots + (size_t)m * RBLK);
+    multi_dot_partial<<<dim3(RBLK, (m + 3) / 4), RB, 0, stream>>>(A, lda, m, x, n, dots);
+    multi_dot_final<<<m, 128, 0, stream>>>(dots, 1.0, dots + (size_t)m * RBLK);
     launch_count += 2;
     TCI_CUDA(cudaGetLastError());
     TCI_CUDA(cudaMemcpyAsync(host_out, dots + (size_t)m * RBLK, m * sizeof(double), cudaMemcpyDeviceToHost, stream));
@@ -2185,7 +2205,7 @@ struct tci_ctx {
   // device-resident single dot into dots[off]
   void dot_dev(const double* a, const double* x, i64 n, double* dev_out) {
     multi_dot_partial<<<RBLK, RB, 0, stream>>>(a, 0, 1, x, n, dots);
-    multi_dot_final<<<1, 32, 0, stream>>>(dots, 1, RBLK, dev_out);
+    multi_dot_final<<<1, 128, 0, stream>>>(dots, 1.0, dev_out);
     launch_count += 2;
     TCI_CUDA(cudaGetLastError());
   }
@@ -3039,6 +3059,7 @@ std::unique_ptr<tci_ctx> new_ctx(int64_t device) {
   TCI_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   TCI_CUDA(cudaEventCreate(&ctx->ev0));
   TCI_CUDA(cudaEventCreate(&ctx->ev1));
+  TCI_CUDA(cudaEventCreateWithFlags(&ctx->ev_last, cudaEventDisableTiming));
   return ctx;
 }
 
@@ -3310,6 +3331,12 @@ int ctx_from_plan(CsfSpace&& sp, Plan&& plan, const double* chol, int64_t device
 
 extern "C" {
 
+static bool is_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 int tci_sigma_device(tci_ctx* ctx, const double* d_c, double* d_sigma, int64_t n, void* stream) {
   if (!ctx || !d_c || !d_sigma) return TCI_ERR_ARG;
   try {
@@ -3341,6 +3368,7 @@ int tci_sigma_device(tci_ctx* ctx, const double* d_c, double* d_sigma, int64_t n
     TCI_CUDA(cudaGetLastError());
     TCI_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     TCI_CUDA(cudaStreamWaitEvent(user, ctx->ev1, 0));
+    if (!is_capturing(user)) TCI_CUDA(cudaEventRecord(ctx->ev_last, ctx->stream));
     ctx->sigma_count++;
     return TCI_OK;
   } catch (...) {
@@ -3839,8 +3867,8 @@ int tci_davidson_ex(tci_ctx* ctx, int64_t nroots, double tol_residual, double to
           normalize_kernel<<<G, TB, 0, st>>>(r, dev_ov + 1, n);
           ctx->launch_count++;
           for (int pass = 0; pass < 2 && num_vec > 0; ++pass) {
-            multi_dot_partial<<<RBLK, RB, 0, st>>>(Cs, n, num_vec, r, n, ctx->dots);
-            multi_dot_final_neg<<<(num_vec + 127) / 128, 128, 0, st>>>(ctx->dots, num_vec, RBLK, dev_coef);
+            multi_dot_partial<<<dim3(RBLK, (num_vec + 3) / 4), RB, 0, st>>>(Cs, n, num_vec, r, n, ctx->dots);
+            multi_dot_final<<<num_vec, 128, 0, st>>>(ctx->dots, -1.0, dev_coef);
             lincomb_kernel<<<G, TB, 0, st>>>(r, 1.0, Cs, dev_coef, nullptr, nullptr, num_vec, n, n);
             ctx->launch_count += 3;
           }
@@ -3933,9 +3961,9 @@ int tci_dots(tci_ctx* ctx, const double* d_A, int64_t lda, int64_t m, const doub
   try {
     TCI_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t user = stream ? (cudaStream_t)stream : cudaStreamLegacy;
-    const int64_t need = m * (RBLK + 1);
+    const int64_t need = m * RBLK;
     if (need > ctx->dotbuf_cap) {
-      TCI_CUDA(cudaStreamSynchronize(ctx->stream));
+      TCI_CUDA(cudaStreamSynchronize(ctx->stream));  // the last call too: the stream waits for it
       if (ctx->dotbuf) {
         std::lock_guard<std::mutex> lk(g_capture_free_mu);
         TCI_CUDA(dev_free(ctx->dotbuf, ctx->stream));
@@ -3946,16 +3974,29 @@ int tci_dots(tci_ctx* ctx, const double* d_A, int64_t lda, int64_t m, const doub
         cudaGetLastError();
         throw Error(TCI_ERR_MEMORY, "device allocation of the projection scratch failed");
       }
+      TCI_CUDA(cudaStreamSynchronize(ctx->stream));  // the caller's stream may use it
       ctx->dotbuf_cap = need;
     }
-    TCI_CUDA(cudaEventRecord(ctx->ev0, user));
-    TCI_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev0, 0));
-    multi_dot_partial<<<RBLK, RB, 0, ctx->stream>>>(d_A, lda, (int)m, d_x, n, ctx->dotbuf);
-    multi_dot_final<<<(unsigned)((m + 127) / 128), 128, 0, ctx->stream>>>(ctx->dotbuf, (int)m, RBLK, d_out);
+    // A capturing caller forks to the context's stream and joins it again.  Otherwise the kernels run on the caller's
+    // stream, after the context's last device work (ev_last) and before its next: back-to-back calls on one stream
+    // then cross to no other stream.
+    const bool fork = is_capturing(user);
+    cudaStream_t run = fork ? ctx->stream : user;
+    if (fork) {
+      TCI_CUDA(cudaEventRecord(ctx->ev0, user));
+      TCI_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev0, 0));
+    } else {
+      TCI_CUDA(cudaStreamWaitEvent(user, ctx->ev_last, 0));
+    }
+    // about a thousand elements a block, at most the scratch's RBLK blocks a row
+    const int nblk = (int)std::min<int64_t>(RBLK, (n + 1023) / 1024);
+    multi_dot_partial<<<dim3((unsigned)nblk, (unsigned)((m + 3) / 4)), RB, 0, run>>>(d_A, lda, (int)m, d_x, n, ctx->dotbuf);
+    dots_final<<<(unsigned)m, 32, 0, run>>>(ctx->dotbuf, nblk, d_out);
     ctx->launch_count += 2;
     TCI_CUDA(cudaGetLastError());
-    TCI_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
-    TCI_CUDA(cudaStreamWaitEvent(user, ctx->ev1, 0));
+    cudaEvent_t done = fork ? ctx->ev0 : ctx->ev_last;
+    TCI_CUDA(cudaEventRecord(done, run));
+    TCI_CUDA(cudaStreamWaitEvent(fork ? user : ctx->stream, done, 0));
     return TCI_OK;
   } catch (...) {
     return guard_status(std::current_exception());

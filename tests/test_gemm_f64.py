@@ -42,3 +42,21 @@ def test_gemm_against_numpy(tA, tB, pad, off, need_gpu):
             # either side
             assert (np.abs(got[:, :N] - ref) <= 2 * (nseg * K + 4) * 2.0 ** -53 * mag).all(), (M, N, K, nseg)
             assert (got[:, N:] == C2[:, N:]).all()
+
+
+@pytest.mark.parametrize("K", [3, 16, 70])
+def test_many_segments(K, need_gpu):
+    """Segment counts around the 16 records a block holds at a time and around twice that, tiles of 2 x 2 to 8 x 16
+    blocks."""
+    rng = np.random.default_rng(K)
+    for M, N in ((16, 16), (35, 33), (53, 57), (64, 128), (200, 300)):
+        for nseg in (2, 15, 16, 17, 31, 32, 33, 50):
+            A, B, C = (rng.uniform(-0.5, 0.5, s) for s in (nseg * M * K, nseg * K * N, M * N))
+            got = C.copy()
+            rc = lib().tci_selftest_gemm_f64(0, M, N, K, nseg, 0, 0, K, N, N, 0, 0, M * K, K * N, 0.5, 1.0, ptr(A), A.size,
+                                             ptr(B), B.size, ptr(got))
+            assert rc == 0
+            A3, B3 = A.reshape(nseg, M, K), B.reshape(nseg, K, N)
+            ref = C.reshape(M, N) + 0.5 * np.einsum("smk,skn->mn", A3, B3, optimize=True)
+            mag = np.abs(C.reshape(M, N)) + 0.5 * np.einsum("smk,skn->mn", np.abs(A3), np.abs(B3), optimize=True)
+            assert (np.abs(got.reshape(M, N) - ref) <= 2 * (nseg * K + 4) * 2.0 ** -53 * mag).all(), (M, N, nseg)

@@ -10,9 +10,13 @@
 // copies and barriers run under the other's products; four 16-deep slices in flight by cp.async. Measured on a B200:
 // 592 problems of 256 x 256 x (40 x 256) 31 TFLOP/s, 576 of 173 x 173 x (40 x 173) 23 (6 % of the blocks padding,
 // uneven column shares; 20 with one body for all shapes and predicates for the missing blocks). Against the scalar
-// kernels: two-external step at 24 pairs x 173 virtuals 102 -> 35 ms, all-external at 240 virtuals 6.8 -> 5.1 ms. Tried and slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp
-// that only copies (registers spill at two blocks per SM), the copies dealt between the products (the loop outgrows
-// the instruction cache: 9-17).
+// kernels: two-external step at 24 pairs x 173 virtuals 102 -> 35 ms, all-external at 240 virtuals 6.8 -> 5.1 ms. Tried and
+// slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers spill at two blocks per
+// SM), the copies dealt between the products (the loop outgrows the instruction cache: 9-17).
+//
+// A launch of few tiles is bound by the latency of a slice (copy, barrier, products: 1.3 us), one after another: there
+// eight warps share 64-deep slices of tiles down to 16 x 16. 32 problems of 35 x 35 x (40 x 35): 76 us with four
+// warps, 32-deep slices and 64-row tiles, 48 us so; 64 of 53 x 53 x (40 x 53): 98 -> 83 us.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -29,7 +33,8 @@ namespace {
 using tci_dev::DGemmProblem;
 using tci_dev::DGemmSeg;
 
-constexpr int NT = 128;  // four warps
+// Threads of a block: four warps side by side on a tile's columns, or eight sharing k (WK).
+constexpr int threads(int wk) { return wk == 1 ? 128 : 256; }
 
 __device__ __forceinline__ void cp_async16(unsigned s, const void* g, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(bytes) : "memory");
@@ -62,7 +67,7 @@ __device__ __forceinline__ unsigned chunk(int c0, int c1, int sw) {
 // the banks).  16-byte copies want a 16-byte aligned operand with an even leading dimension.
 enum Mode { K16, K8, RT8, R8, R16 };
 
-template <int R, int BK, Mode M>
+template <int R, int BK, Mode M, int NT>
 struct Operand {
   static constexpr int RP = R <= 8 ? 8 : R <= 16 ? 16 : R <= 32 ? 32 : R <= 64 ? 64 : 128;
   static constexpr bool KROWS = M == R16, KC = M == K16 || M == K8;
@@ -139,33 +144,33 @@ struct Operand {
 };
 
 // MB: 8-row blocks of a tile.  WK = 1: the four warps share a tile's columns (up to 16 blocks of 8, dealt evenly),
-// 16-deep k slices; WK = 4: each warp takes a quarter of every 32-deep slice over the whole tile (up to 4 column
-// blocks) and the four sums are added in warp order at the end.  Tiles are cut evenly in 8-row / 8-column blocks (a
+// 16-deep k slices; WK = 8: eight warps, each takes 8 of every 64-deep slice over the whole tile (up to 4 column
+// blocks), and the eight sums are added in warp order at the end.  Tiles are cut evenly in 8-row / 8-column blocks (a
 // 173-row problem gives 64 + 56 + 56 rows, not 64 + 64 + 45); blocks past the edge are not computed.
 constexpr int NB = 4;  // column blocks of a warp at most
 template <int MB, int WK, Mode AM, Mode BM_>
 struct Shape {
-  static constexpr int BK = WK == 1 ? 16 : 32;
+  static constexpr int NT = threads(WK), BK = WK == 1 ? 16 : 64;
   static constexpr int BM = 8 * MB, BN = 8 * NB * (WK == 1 ? 4 : 1);
-  using A = Operand<BM, BK, AM>;
-  using B = Operand<(WK == 4 && BM_ == R16 ? BN + 8 : BN), BK, BM_>;  // room for a shifted row
+  using A = Operand<BM, BK, AM, NT>;
+  using B = Operand<(WK > 1 && BM_ == R16 ? BN + 8 : BN), BK, BM_, NT>;  // room for a shifted row
   static constexpr int STAGE = A::SIZE + B::SIZE;  // doubles
   static constexpr int STG = 4;
   static constexpr size_t smem = sizeof(double) * (size_t)STAGE * STG;
 };
 
 template <int MB, int WK, Mode AM, Mode BM_>
-__global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
+__global__ void __launch_bounds__(threads(WK), WK == 1 ? 2 : 1) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
                                                       const DGemmSeg* __restrict__ segs) {
   using Sh = Shape<MB, WK, AM, BM_>;
-  constexpr int BK = Sh::BK, STG = Sh::STG;
+  constexpr int NT = Sh::NT, BK = Sh::BK, STG = Sh::STG;
   constexpr bool KB = Sh::B::KROWS;
   extern __shared__ __align__(128) double sm[];
   __shared__ double meta_alpha[STG];
   __shared__ int meta_k[STG];  // valid k of the slice; + 256: alpha is not 1; + 512, 1024: shifts of even, odd k
   const int lane = threadIdx.x & 31;
   // rotated: the uneven shares fall on every scheduler in turn
-  const int role = ((threadIdx.x >> 5) + blockIdx.x) & 3;
+  const int role = WK == 1 ? ((threadIdx.x >> 5) + blockIdx.x) & 3 : threadIdx.x >> 5;
   // the problem of this tile (the last with tile_begin <= tile), 32 probes at a time
   const long long tile = blockIdx.x;
   int lo = 0, cnt = nprob;
@@ -177,10 +182,10 @@ __global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __rest
     cnt = min(step, cnt - c * step);
   }
   const DGemmProblem P = probs[lo];
-  const bool tr = P.trans_c != 0;
+  const bool tr = (P.trans_c & 1) != 0;
   const long long rows = tr ? P.N : P.M, cols = tr ? P.M : P.N;
   const int tn = (int)P.tiles_n, t = (int)(tile - P.tile_begin), ti = t / tn, tj = t % tn;
-  const int mblk = (int)((rows + 7) >> 3), nblk = (int)((cols + 7) >> 3), tm = (mblk + 7) >> 3;
+  const int mblk = (int)((rows + 7) >> 3), nblk = (int)((cols + 7) >> 3), tm = (int)(P.trans_c >> 1);
   const int mq = mblk / tm, mr = mblk % tm, nq = nblk / tn, nr = nblk % tn;
   const long long m0 = 8ll * (ti * mq + min(ti, mr)), n0 = 8ll * (tj * nq + min(tj, nr));
   const int mb = mq + (ti < mr ? 1 : 0), nbt = nq + (tj < nr ? 1 : 0);  // mb: MB or MB - 1
@@ -203,14 +208,27 @@ __global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __rest
   double alpha = 1.0;
   typename Sh::A oa;
   typename Sh::B ob;
-  DGemmSeg S{};
-  if (sg < sge) S = segs[sg];
-  auto open = [&]() {  // segment sg (loaded earlier), and the load of the one after it
+  // the segment records, RING ahead, by cp.async with the slices (a record loaded at its use cost a short segment's
+  // slice its latency again)
+  constexpr int RING = 16, WORDS = sizeof(DGemmSeg) / 8;
+  static_assert(sizeof(DGemmSeg) == 8 * WORDS && RING * WORDS <= NT, "records by 8-byte words");
+  __shared__ __align__(8) double ring[RING * WORDS];
+  if ((int)threadIdx.x < RING * WORDS && sg + (int)threadIdx.x / WORDS < sge)
+    ring[threadIdx.x] = reinterpret_cast<const double*>(segs + sg)[threadIdx.x];
+  __syncthreads();
+  const unsigned rbase = static_cast<unsigned>(__cvta_generic_to_shared(ring));
+  int rs = 0;  // the place of segment sg
+  auto open = [&]() {
+    const DGemmSeg& S = *reinterpret_cast<const DGemmSeg*>(ring + rs * WORDS);
     krem = (int)S.K;
     alpha = S.alpha;
     oa.open(tr ? S.B : S.A, tr ? S.ldb : S.lda, m0);
     flags = 512 * ob.open(tr ? S.A : S.B, tr ? S.lda : S.ldb, n0) + (alpha != 1.0 ? 256 : 0);
-    if (sg + 1 < sge) S = segs[sg + 1];
+    // the record RING - 1 ahead takes the place of the one before this, which everyone has left
+    const int ahead = sg + RING - 1, pl = rs == 0 ? RING - 1 : rs - 1;
+    if (sg > (int)P.seg_begin && ahead < sge && (int)threadIdx.x < WORDS)
+      cp_async8(rbase + 8u * (unsigned)(pl * WORDS + threadIdx.x), reinterpret_cast<const double*>(segs + ahead) + threadIdx.x, 8);
+    rs = rs == RING - 1 ? 0 : rs + 1;
   };
   if (sg < sge) open();
   auto produce = [&](int st) {
@@ -230,7 +248,10 @@ __global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __rest
     cp_commit();
   };
 #pragma unroll 1
-  for (int st = 0; st < STG - 1; ++st) produce(st);
+  for (int st = 0; st < STG - 1; ++st) {
+    __syncthreads();  // a record's place is refilled one segment after its use
+    produce(st);
+  }
   // fragment addresses: lane (g, tq) holds row g of a block at k = 4 s + tq of step s; with k contiguous, step s's
   // chunks 2 s, 2 s + 1 of a row's 8
   const int f0 = g * BK + 2 * ((tq >> 1) ^ swz(g)) + (tq & 1);
@@ -308,12 +329,12 @@ __global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __rest
 #pragma unroll
       for (int j = 0; j < NB; ++j) red[(role * MB * NB + i * NB + j) * 32 + lane] = make_double2(acc[i][j][0], acc[i][j][1]);
     __syncthreads();
-    for (int e = role; e < MB * NB; e += 4) {
+    for (int e = role; e < MB * NB; e += WK) {
       const int i = e / NB, j = e % NB;
       if (i >= mb || j >= nb) continue;
       double2 v = red[e * 32 + lane];
 #pragma unroll
-      for (int w = 1; w < 4; ++w) {
+      for (int w = 1; w < WK; ++w) {
         const double2 x = red[(w * MB * NB + e) * 32 + lane];
         v.x += x.x;
         v.y += x.y;
@@ -326,7 +347,7 @@ __global__ void __launch_bounds__(NT, 2) gemm_mma_f64(const DGemmProblem* __rest
 template <int MB, int WK, Mode AM, Mode BM_>
 cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles, cudaStream_t st) {
   constexpr size_t smem = Shape<MB, WK, AM, BM_>::smem;
-  static_assert(WK == 1 || smem >= sizeof(double2) * 4 * MB * NB * 32, "the warps' sums fit the stages");
+  static_assert(WK == 1 || smem >= sizeof(double2) * WK * MB * NB * 32, "the warps' sums fit the stages");
   static std::once_flag once[64];  // the attribute, once per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -335,7 +356,7 @@ cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long 
   std::call_once(once[dev], [&] {
     cudaFuncSetAttribute(gemm_mma_f64<MB, WK, AM, BM_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
-  gemm_mma_f64<MB, WK, AM, BM_><<<(unsigned)ntiles, NT, smem, st>>>(probs, nprob, segs);
+  gemm_mma_f64<MB, WK, AM, BM_><<<(unsigned)ntiles, threads(WK), smem, st>>>(probs, nprob, segs);
   return cudaGetLastError();
 }
 
@@ -343,22 +364,22 @@ using Go = cudaError_t (*)(const DGemmProblem*, int, const DGemmSeg*, long long,
 #define TCI_ROWS(WK, A, B) \
   go<1, WK, A, B>, go<2, WK, A, B>, go<3, WK, A, B>, go<4, WK, A, B>, go<5, WK, A, B>, go<6, WK, A, B>, go<7, WK, A, B>, \
       go<8, WK, A, B>
-#define TCI_PAIR(A, B) TCI_ROWS(1, A, B), TCI_ROWS(4, A, B)
+#define TCI_PAIR(A, B) TCI_ROWS(1, A, B), TCI_ROWS(8, A, B)
 constexpr Go kGo[tci_dmma::CLASSES] = {TCI_PAIR(K16, K16), TCI_PAIR(K16, R16), TCI_PAIR(K8, K8),
                                        TCI_PAIR(K8, R16),  TCI_PAIR(RT8, K8),  TCI_PAIR(RT8, R16)};
 #undef TCI_PAIR
 #undef TCI_ROWS
 
-// Tile counts of a problem of rows x cols: at most 8 row blocks x bnb column blocks (the warps sharing k: 8 x 4).
+// Tile counts of a problem of rows x cols: at most bmb row blocks x bnb column blocks.
 struct Cut {
   long long tm, tn;
   int mb, nb;   // blocks of its largest tile
   double cost;  // 8 x 8 blocks computed, each tile's slowest warp times four
 };
-Cut cut(long long rows, long long cols, int bnb) {
+Cut cut(long long rows, long long cols, int bmb, int bnb) {
   const long long mblk = (rows + 7) / 8, nblk = (cols + 7) / 8;
   Cut c;
-  c.tm = (mblk + 7) / 8;
+  c.tm = (mblk + bmb - 1) / bmb;
   c.tn = (nblk + bnb - 1) / bnb;
   c.mb = (int)((mblk + c.tm - 1) / c.tm);
   c.nb = (int)((nblk + c.tn - 1) / c.tn);
@@ -366,37 +387,47 @@ Cut cut(long long rows, long long cols, int bnb) {
   return c;
 }
 
-// Adds a problem to the class its operands and tile allow; bnb = NB: the warps share k.  *work: the largest tile's
-// blocks x the problem's k.
-void add_problem(const DGemmProblem& g, const std::vector<DGemmSeg>& segs, int bnb, tci_dmma::Tiles& t, double& work) {
-  DGemmProblem x = g;
-  x.trans_c = cut(g.N, g.M, bnb).cost < 0.8 * cut(g.M, g.N, bnb).cost ? 1 : 0;
-  bool row_k = true, row_r = true, col_k = true, col_r = true, row_even = true, col_even = true;
+// What the segments of a problem have in common, of either operand: storage order, room for 16-byte copies.
+struct Form {
+  bool a_k = true, a_r = true, b_k = true, b_r = true, a_even = true, b_even = true;
   double k = 0;
+};
+Form form(const DGemmProblem& g, const std::vector<DGemmSeg>& segs) {
+  Form f;
   for (long long q = g.seg_begin; q < g.seg_end; ++q) {
     const DGemmSeg& y = segs[(size_t)q];
-    const bool rk = x.trans_c ? y.tB != 0 : y.tA == 0, ck = x.trans_c ? y.tA == 0 : y.tB != 0;
-    row_k = row_k && rk;
-    row_r = row_r && !rk;
-    col_k = col_k && ck;
-    col_r = col_r && !ck;
-    const bool ea = (y.lda & 1) == 0 && (reinterpret_cast<uintptr_t>(y.A) & 15) == 0;
-    const bool eb = (y.ldb & 1) == 0 && (reinterpret_cast<uintptr_t>(y.B) & 15) == 0;
-    row_even = row_even && (x.trans_c ? eb : ea);
-    col_even = col_even && (x.trans_c ? ea : eb);
-    k += (double)y.K;
+    f.a_k = f.a_k && y.tA == 0;
+    f.a_r = f.a_r && y.tA != 0;
+    f.b_k = f.b_k && y.tB != 0;
+    f.b_r = f.b_r && y.tB == 0;
+    f.a_even = f.a_even && (y.lda & 1) == 0 && (reinterpret_cast<uintptr_t>(y.A) & 15) == 0;
+    f.b_even = f.b_even && (y.ldb & 1) == 0 && (reinterpret_cast<uintptr_t>(y.B) & 15) == 0;
+    f.k += (double)y.K;
   }
-  if ((!row_k && !row_r) || (!col_k && !col_r))
+  if ((!f.a_k && !f.a_r) || (!f.b_k && !f.b_r))
     throw std::invalid_argument("a GEMM problem whose segments differ in storage order");
+  return f;
+}
+
+// Tiles and class of a problem at a largest tile of bmb x bnb blocks; bnb <= NB: the warps share k.
+struct Place {
+  bool swapped;
+  Cut c;
+  int cls;
+  double work;  // its largest tile's blocks x its k (k-sharing: four blocks' worth for what a slice costs besides)
+};
+Place place(const DGemmProblem& g, const Form& f, int bmb, int bnb) {
+  Place x;
+  x.swapped = cut(g.N, g.M, bmb, bnb).cost < 0.8 * cut(g.M, g.N, bmb, bnb).cost;
+  // rows and columns of the tiles, in terms of C^T = B^T A^T when the operands change places
+  const bool row_k = x.swapped ? f.b_k : f.a_k, col_k = x.swapped ? f.a_k : f.b_k;
+  const bool row_even = x.swapped ? f.b_even : f.a_even, col_even = x.swapped ? f.a_even : f.b_even;
   if (!col_k && !col_even && bnb > NB) bnb = std::min(bnb, 15);  // room for shifted rows
-  const Cut c = x.trans_c ? cut(g.N, g.M, bnb) : cut(g.M, g.N, bnb);
+  x.c = x.swapped ? cut(g.N, g.M, bmb, bnb) : cut(g.M, g.N, bmb, bnb);
   const int modes = !row_k ? (col_k ? 4 : 5) : col_k ? (row_even && col_even ? 0 : 2) : (row_even ? 1 : 3);
-  const int cls = c.mb - 1 + (bnb <= NB ? 8 : 0) + 16 * modes;
-  x.tiles_n = c.tn;
-  x.tile_begin = t.ntiles[cls];
-  t.ntiles[cls] += c.tm * c.tn;
-  t.probs[cls].push_back(x);
-  work = std::max(work, (double)c.mb * (bnb <= NB ? c.nb : (c.nb + 3) / 4 * 4) * k);
+  x.cls = x.c.mb - 1 + (bnb <= NB ? 8 : 0) + 16 * modes;
+  x.work = (bnb <= NB ? (double)x.c.mb * x.c.nb + 4 : (double)x.c.mb * ((x.c.nb + 3) / 4 * 4)) * f.k;
+  return x;
 }
 
 }  // namespace
@@ -405,33 +436,49 @@ namespace tci_dmma {
 
 Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& segs) {
   // the longest problems first: the short ones fill the last wave
-  std::vector<std::pair<long long, size_t>> order;
+  std::vector<Form> forms;
+  std::vector<size_t> order;
   for (size_t i = 0; i < pr.size(); ++i) {
-    long long k = 0;
-    for (long long q = pr[i].seg_begin; q < pr[i].seg_end; ++q) k += segs[(size_t)q].K;
-    order.push_back({-k, i});
+    forms.push_back(form(pr[i], segs));
+    order.push_back(i);
   }
-  std::stable_sort(order.begin(), order.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return forms[a].k > forms[b].k; });
   // Tile width by the time the fullest SM would need: waves of tiles x the largest tile, the narrower ones at the
   // rate they were measured at (28 TFLOP/s for 12 blocks, 24 for 8 and 19 for the k-sharing 4 against 30 for 16 on
   // a launch that fills the chip).  Wide tiles win once there are several waves, narrow and k-sharing ones where a
   // launch would leave SMs idle.
   const double sms = (double)tci_dev::device_sms();
-  Tiles best;
+  struct Try {
+    int bmb, bnb;
+    double slow;
+  };
+  Try best{8, 16, 1.0};
   double best_time = 0;
-  for (const auto& [bnb, slow] : {std::pair<int, double>{16, 1.0}, {12, 1.12}, {8, 1.25}, {NB, 1.6}}) {
-    Tiles t;
+  for (const Try& y : {best, Try{8, 12, 1.12}, Try{8, 8, 1.25}, Try{8, NB, 1.6}, Try{4, NB, 1.6}, Try{3, 3, 1.6}, Try{2, 2, 1.6}}) {
     double work = 0, n = 0;
-    for (const auto& o : order) add_problem(pr[o.second], segs, bnb, t, work);
-    for (long long k : t.ntiles) n += (double)k;
-    const double time = std::ceil(n / sms) * work * slow;
-    if (bnb == 16 || time < 0.97 * best_time) {
-      best = std::move(t);
+    for (size_t i = 0; i < pr.size(); ++i) {
+      const Place x = place(pr[i], forms[i], y.bmb, y.bnb);
+      n += (double)(x.c.tm * x.c.tn);
+      work = std::max(work, x.work);
+    }
+    const double time = std::ceil(n / sms) * work * y.slow;
+    if (y.bnb == 16 || time < 0.97 * best_time) {
+      best = y;
       best_time = time;
     }
     if (n > 16 * sms) break;
   }
-  return best;
+  Tiles t;
+  for (size_t i : order) {
+    const Place x = place(pr[i], forms[i], best.bmb, best.bnb);
+    DGemmProblem g = pr[i];
+    g.trans_c = (x.swapped ? 1 : 0) | 2 * x.c.tm;
+    g.tiles_n = x.c.tn;
+    g.tile_begin = t.ntiles[x.cls];
+    t.ntiles[x.cls] += x.c.tm * x.c.tn;
+    t.probs[x.cls].push_back(g);
+  }
+  return t;
 }
 
 cudaError_t launch(const Tables& t, const DGemmSeg* segs, cudaStream_t st) {

@@ -18,7 +18,8 @@ struct DGemmProblem {
   double beta;
   long long seg_begin, seg_end;
   long long trans_c;  // gemm_tc.cu: M, N and the segments describe C^T = B^T A^T;
-                         // gemm_mma_f64.cu: computed with the operands swapped
+                         // gemm_mma_f64.cu: bit 0: computed with the operands swapped, the rest:
+                         // tiles along the rows
 };
 struct DGemmSeg {
   const double* A;

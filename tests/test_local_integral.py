@@ -35,3 +35,17 @@ def test_integral_form_refused_in_mixed_precision(need_gpu):
     _, L = synthetic_operator(15, 10, seed=4)
     with pytest.raises(Exception):
         local.LocalAllExternal(3, 12, L, heads, dom, total, precision="tf32x3", form="integral")
+
+
+def test_integral_form_more_columns_than_a_block_holds(need_gpu):
+    """91 pairs whose domains nearly all hold every external: up to 182 columns for one a, in batches, jobs of several
+    passes and of single columns."""
+    heads, dom, total = local.pair_domain_problem(91, 13, 20, 17, 20, seed=2)
+    _, L = synthetic_operator(33, 30, seed=4, scale=0.5)
+    c = random_civec(total, 3)
+    ref = dense.allext_local_sigma(13, L, heads, dom, c)
+    op = local.LocalAllExternal(13, 20, L, heads, dom, total, form="integral")
+    got = op.apply(c)
+    assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+    assert np.array_equal(got, op.apply(c))
+    op.close()

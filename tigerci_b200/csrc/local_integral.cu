@@ -7,11 +7,15 @@
 // both a and c (a twelfth of them where a domain is 28 % of the externals) are its right-hand sides: C_h[c][:] with
 // zeros outside D_h.  A thread block owns one a and up to 64 rows b, walks the c that occur, multiplies the row's part
 // by its right-hand sides on the FP64 matrix instruction (up to 48 columns at a time, 16-deep slices of d staged by
-// cp.async two ahead) and adds the products to per-column sums in shared memory; b <= a is half of the matrix.  The
-// zero padding inside a column costs 1 / density in d and b, but nothing is gathered: the index arithmetic of a
+// cp.async two ahead) and adds the products to per-column sums in shared memory; b <= a is half of the matrix.  Four
+// warps copy and four multiply, a stage handed over by named barriers: the index arithmetic of the copies (triangular
+// rows, three cases) is most of the instructions, and in the warps that multiply it held the products back (15.4 ms at
+// 150 pairs of 20-150 of 300 externals with eight warps doing both, 13.8 with eight multiplying, 13.5 with four; four
+// stages, or two of 32 k, are no faster: 13.7, 14.4).  The zero
+// padding inside a column costs 1 / density in d and b, but nothing is gathered: the index arithmetic of a
 // gathering kernel (lanes over the domain, integrals from shared memory) cost more than the padding (30 ms against
 // 11 at 150 pairs of 20-150 of 300 externals), and n^2 sum n_h^2 products replace the Cholesky form's 4 nchol sum n_h^3.
-// Bound by the FP64 pipe and by the staging of the rows from L2.  Every sum in a fixed order.
+// Bound by the copies (9.9 ms alone) and the products of half-filled tiles (11.4 alone) together.  Every sum in a fixed order.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -24,7 +28,7 @@ using tci_lint::Block;
 using tci_lint::Job;
 using tci_lint::Task;
 
-constexpr int NT = 256;                    // 4 x 2 warps: up to 16 rows x half of the columns each
+constexpr int NC = 128, NP = 128, NT = NC + NP;  // four warps of up to 16 rows x all columns each, four that copy
 constexpr int ROWS = 64, COLS = 48, BK = 16, STG = 3;
 constexpr int ACC_COLS = 128, YP = ROWS + 4;  // accumulators of a task: columns, pitch
 constexpr int STAGE = (ROWS + COLS) * BK;     // doubles
@@ -42,6 +46,10 @@ __device__ __forceinline__ void mma884(double& c0, double& c1, double a, double 
                : "+d"(c0), "+d"(c1)
                : "d"(a), "d"(b));
 }
+// named barriers: a stage is full (the copying warps arrive, the others wait) or free again (the other way round)
+__device__ __forceinline__ void bar_sync(int id) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(NT) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(NT) : "memory"); }
+constexpr int FULL = 1, FREE = FULL + STG;
 // rows of 16 k as eight 16-byte chunks, chunk c at place c ^ swz(row): as in gemm_mma_f64.cu
 __device__ __forceinline__ int swz(int r) { return ((r & 3) << 1) | ((r >> 2) & 1); }
 __device__ __forceinline__ unsigned place(int r, int k) {  // bytes
@@ -57,137 +65,144 @@ __global__ void __launch_bounds__(NT, 2) local_integral(const Task* __restrict__
   extern __shared__ __align__(128) double sm[];
   double* Y = sm + STG * STAGE;  // [column][row]
   const Task T = tasks[blockIdx.x];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
-  // the four row shares of the tile, rotated so that the uneven ones fall on every scheduler in turn; two column shares
-  const int wm = (warp + (int)blockIdx.x) & 3, wn = warp >> 2;
-  const int mblk = (T.rows + 7) >> 3, i0 = mblk * wm >> 2, mb = (mblk * (wm + 1) >> 2) - i0;  // its 8-row blocks: 0 .. 2
+  const int tid = threadIdx.x;
   for (int i = tid; i < T.ncol * YP; i += NT) Y[i] = 0.0;
-  const unsigned sbase = static_cast<unsigned>(__cvta_generic_to_shared(sm));
-  const int b1 = T.b0 + T.rows, nsl = (nv + BK - 1) / BK;
-  // producer cursor: job, slice; two columns of the job per thread
-  int pj = T.job0, ps = 0, pcnt = 0;
-  const double *prow = nullptr, *pc0 = nullptr, *pc1 = nullptr;
-  const int bj = tid >> 3, bk = 2 * (tid & 7);  // this thread's column (and + 32) and k of a 16-byte copy
-  auto open = [&]() {
-    const Job J = jobs[pj];
-    pcnt = J.cnt;
-    prow = X + (long long)tri(T.a, J.c) * npv;
-    if (bj < pcnt) pc0 = C + ((long long)cblk[T.col0 + jcol[J.off + bj]] * nv + J.c) * ldc + bk;
-    if (bj + 32 < pcnt) pc1 = C + ((long long)cblk[T.col0 + jcol[J.off + bj + 32]] * nv + J.c) * ldc + bk;
-  };
-  if (pj < T.job1) open();
-  // this thread's copies of a slice: rows r0, r0 + 16, ... at one k where the integrals of a row b lie along d <= b,
-  // row ru at k0, k0 + 4, ... where those of one d lie along b
-  const int kl = tid & 15, r0 = tid >> 4, ru = tid & 63, k0 = tid >> 6;
-  int offl[4];
-  unsigned pl[4];
+  __syncthreads();
+  const int nsl = (nv + BK - 1) / BK, total_sl = (T.job1 - T.job0) * nsl;
+  if (tid >= NC) {
+    // copying warps: job by job, slice by slice
+    const int pt = tid - NC, b1 = T.b0 + T.rows;
+    const unsigned sbase = static_cast<unsigned>(__cvta_generic_to_shared(sm));
+    // this thread's copies of a slice: rows r0, r0 + 8, ... at one k where the integrals of a row b lie along d <= b,
+    // row ru at k0, k0 + 2, ... where those of one d lie along b; 16 bytes of up to three columns of the job
+    const int kl = pt & 15, r0 = pt >> 4, ru = pt & 63, k0 = pt >> 6, bj = pt >> 3, bk = 2 * (pt & 7);
+    int offl[8];
+    unsigned pl[8];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    offl[u] = tri(T.b0 + r0 + 16 * u, 0) + kl;
-    pl[u] = place(ru, k0 + 4 * u);
-  }
-  const unsigned pk = place(r0, kl), pb0 = place(bj, bk), pb1 = place(bj + 32, bk);
-  auto produce = [&](int st) {
-    if (pj < T.job1) {
-      const unsigned s = sbase + 8u * (unsigned)(st * STAGE), sb = s + 8u * (unsigned)(ROWS * BK);
-      const int d0 = ps * BK;
-      if (d0 + BK <= T.b0 + 1) {  // d <= b throughout
-        const double* q = prow + d0;
+    for (int u = 0; u < 8; ++u) {
+      offl[u] = tri(T.b0 + r0 + 8 * u, 0) + kl;
+      pl[u] = place(ru, k0 + 2 * u);
+    }
+    const unsigned pk = place(r0, kl), pb = place(bj, bk);
+    int st = 0, i = 0;
+    for (int j = T.job0; j < T.job1; ++j) {
+      const Job J = jobs[j];
+      const double* prow = X + (long long)tri(T.a, J.c) * npv;
+      const double* pc[3];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (r0 + 16 * u < T.rows) cp_async8(s + pk + 8u * (16 * u * BK), q + offl[u], 8);
-      } else if (d0 >= b1) {  // d above every b
-        if (ru < T.rows) {
-          const int d = d0 + k0;
-          int o = d * (d + 1) / 2 + T.b0 + ru;
+      for (int u = 0; u < 3; ++u)
+        if (bj + 16 * u < J.cnt) pc[u] = C + ((long long)cblk[T.col0 + jcol[J.off + bj + 16 * u]] * nv + J.c) * ldc + bk;
+      for (int d0 = 0; d0 < nsl * BK; d0 += BK, ++i) {
+        if (i >= STG) bar_sync(FREE + st);
+        const unsigned s = sbase + 8u * (unsigned)(st * STAGE), sb = s + 8u * (unsigned)(ROWS * BK);
+        if (d0 + BK <= T.b0 + 1) {  // d <= b throughout
+          const double* q = prow + d0;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const bool ok = d + 4 * u < nv;
-            cp_async8(s + pl[u], prow + (ok ? o : 0), ok ? 8 : 0);
-            o += 4 * (d + 4 * u) + 10;
+          for (int u = 0; u < 8; ++u)
+            if (r0 + 8 * u < T.rows) cp_async8(s + pk + 8u * (8 * u * BK), q + offl[u], 8);
+        } else if (d0 >= b1) {  // d above every b
+          if (ru < T.rows) {
+            const int d = d0 + k0;
+            int o = d * (d + 1) / 2 + T.b0 + ru;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const bool ok = d + 2 * u < nv;
+              cp_async8(s + pl[u], prow + (ok ? o : 0), ok ? 8 : 0);
+              o += 2 * (d + 2 * u) + 3;
+            }
           }
-        }
-      } else {
-        const int d = d0 + kl;
-        const bool ok = d < nv;
+        } else {
+          const int d = d0 + kl;
+          const bool ok = d < nv;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (r0 + 16 * u < T.rows)
-            cp_async8(s + pk + 8u * (16 * u * BK), prow + (ok ? tri(T.b0 + r0 + 16 * u, d) : 0), ok ? 8 : 0);
-      }
-      if (bj < pcnt) cp_async16(sb + pb0, pc0 + d0);
-      if (bj + 32 < pcnt) cp_async16(sb + pb1, pc1 + d0);
-      if (++ps == nsl) {
-        ps = 0;
-        if (++pj < T.job1) open();
+          for (int u = 0; u < 8; ++u)
+            if (r0 + 8 * u < T.rows)
+              cp_async8(s + pk + 8u * (8 * u * BK), prow + (ok ? tri(T.b0 + r0 + 8 * u, d) : 0), ok ? 8 : 0);
+        }
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (bj + 16 * u < J.cnt) cp_async16(sb + pb + 8u * (16 * u * BK), pc[u] + d0);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        if (i > 0) {
+          asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+          bar_arrive(FULL + (st == 0 ? STG - 1 : st - 1));  // the slice before
+        }
+        st = st == STG - 1 ? 0 : st + 1;
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  for (int st = 0; st < STG - 1; ++st) produce(st);
-  const int f0 = g * BK + 2 * ((tq >> 1) ^ swz(g)) + (tq & 1);  // step s: ^ (s << 2)
-  int st = 0;
-  for (int j = T.job0; j < T.job1; ++j) {
-    const Job J = jobs[j];
-    const int nbk = (J.cnt + 7) >> 3, h0 = (nbk + 1) >> 1;  // column blocks, the first half's
-    const int j0 = wn ? h0 : 0, nb = wn ? nbk - h0 : h0;
-    int col[3][2];  // accumulator columns of this lane's sums
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (total_sl > 0) bar_arrive(FULL + (st == 0 ? STG - 1 : st - 1));
+  } else {
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    // the four row shares of the tile, rotated so that the uneven ones fall on every scheduler in turn; two column shares
+    const int wm = (warp + (int)blockIdx.x) & 3;
+    const int mblk = (T.rows + 7) >> 3, i0 = mblk * wm >> 2, mb = (mblk * (wm + 1) >> 2) - i0;  // its 8-row blocks: 0 .. 2
+    const int f0 = g * BK + 2 * ((tq >> 1) ^ swz(g)) + (tq & 1);  // step s: ^ (s << 2)
+    int st = 0, i = 0;
+    Job next = jobs[T.job0];
+    for (int j = T.job0; j < T.job1; ++j) {
+      const Job J = next;
+      if (j + 1 < T.job1) next = jobs[j + 1];
+      const int nb = (J.cnt + 7) >> 3;  // column blocks
+      int col[6][2];  // accumulator columns of this lane's sums
 #pragma unroll
-    for (int q = 0; q < 3; ++q)
+      for (int q = 0; q < 6; ++q)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int x = 8 * (j0 + q) + 2 * tq + e;
-        col[q][e] = q < nb && x < J.cnt ? jcol[J.off + x] : -1;
-      }
-    double acc[2][3][2];
+        for (int e = 0; e < 2; ++e) {
+          const int x = 8 * q + 2 * tq + e;
+          col[q][e] = x < J.cnt ? jcol[J.off + x] : -1;
+        }
+      double acc[2][6][2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int q = 0; q < 3; ++q) acc[i][q][0] = acc[i][q][1] = 0.0;
-    for (int sl = 0; sl < nsl; ++sl) {
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(STG - 2) : "memory");
-      __syncthreads();  // the slice is there, and the stage refilled below is no longer read
-      produce(st == 0 ? STG - 1 : st - 1);
-      const double* as = sm + st * STAGE + 8 * i0 * BK;
-      const double* bs = sm + st * STAGE + ROWS * BK + 8 * j0 * BK;
-      // one body per number of column blocks: a matrix instruction whose predicate is off still takes its pipe slot
-      auto body = [&](auto rr, auto nn) {
-        constexpr int R = decltype(rr)::value, N = decltype(nn)::value;
+        for (int q = 0; q < 6; ++q) acc[r][q][0] = acc[r][q][1] = 0.0;
+      for (int sl = 0; sl < nsl; ++sl, ++i) {
+        bar_sync(FULL + st);
+        const double* as = sm + st * STAGE + 8 * i0 * BK;
+        const double* bs = sm + st * STAGE + ROWS * BK;
+        // one body per number of column blocks: a matrix instruction whose predicate is off still takes its pipe slot
+        auto body = [&](auto rr, auto nn) {
+          constexpr int R = decltype(rr)::value, N = decltype(nn)::value;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const int fo = f0 ^ (s << 2);
-          double x[R];
+          for (int s = 0; s < 4; ++s) {
+            const int fo = f0 ^ (s << 2);
+            double x[R];
 #pragma unroll
-          for (int i = 0; i < R; ++i) x[i] = as[i * 8 * BK + fo];
+            for (int r = 0; r < R; ++r) x[r] = as[r * 8 * BK + fo];
 #pragma unroll
-          for (int q = 0; q < N; ++q) {
-            const double b = bs[q * 8 * BK + fo];
+            for (int q = 0; q < N; ++q) {
+              const double b = bs[q * 8 * BK + fo];
 #pragma unroll
-            for (int i = 0; i < R; ++i) mma884(acc[i][q][0], acc[i][q][1], x[i], b);
+              for (int r = 0; r < R; ++r) mma884(acc[r][q][0], acc[r][q][1], x[r], b);
+            }
           }
-        }
-      };
-      auto bodies = [&](auto rr) {
-        if (nb == 3) body(rr, std::integral_constant<int, 3>());
-        else if (nb == 2) body(rr, std::integral_constant<int, 2>());
-        else if (nb == 1) body(rr, std::integral_constant<int, 1>());
-      };
-      if (mb == 2) bodies(std::integral_constant<int, 2>());
-      else if (mb == 1) bodies(std::integral_constant<int, 1>());
-      st = st == STG - 1 ? 0 : st + 1;
+        };
+        auto bodies = [&](auto rr) {
+          if (nb == 3) body(rr, std::integral_constant<int, 3>());
+          else if (nb == 4) body(rr, std::integral_constant<int, 4>());
+          else if (nb == 5) body(rr, std::integral_constant<int, 5>());
+          else if (nb == 6) body(rr, std::integral_constant<int, 6>());
+          else if (nb == 2) body(rr, std::integral_constant<int, 2>());
+          else if (nb == 1) body(rr, std::integral_constant<int, 1>());
+        };
+        if (mb == 2) bodies(std::integral_constant<int, 2>());
+        else if (mb == 1) bodies(std::integral_constant<int, 1>());
+        if (i + STG < total_sl) bar_arrive(FREE + st);
+        st = st == STG - 1 ? 0 : st + 1;
+      }
+      // into the columns' sums: the next job's writer of a column is at least one barrier later
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (col[q][e] >= 0) {
+            double* y = Y + col[q][e] * YP + 8 * i0 + g;
+            if (mb > 0) y[0] += acc[0][q][e];
+            if (mb > 1) y[8] += acc[1][q][e];
+          }
     }
-    // into the columns' sums: the next job's writer of a column is at least one barrier later
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        if (col[q][e] >= 0) {
-          double* y = Y + col[q][e] * YP + 8 * i0 + g;
-          if (mb > 0) y[0] += acc[0][q][e];
-          if (mb > 1) y[8] += acc[1][q][e];
-        }
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
   double* out = sigma + T.part * total;
   for (int e = tid; e < T.ncol * ROWS; e += NT) {
@@ -276,8 +291,10 @@ void make_plan(int nv, int nheads, const std::vector<int>& dom, std::vector<Bloc
   double rows_total = 0;
   for (int a = nv - 1; a >= 0; --a) {  // the longest rows first
     const auto& L = of[(size_t)a];
-    for (size_t l0 = 0; l0 < L.size(); l0 += ACC_COLS) {
-      const int ncol = (int)std::min<size_t>(ACC_COLS, L.size() - l0);
+    const size_t nbt = (L.size() + ACC_COLS - 1) / ACC_COLS;  // batches of even width
+    for (size_t x = 0; x < nbt; ++x) {
+      const size_t l0 = L.size() * x / nbt;
+      const int ncol = (int)(L.size() * (x + 1) / nbt - l0);
       Batch bt{a, (int)P.cblk.size(), ncol, (int)P.jobs.size(), 0};
       for (auto& v : by_c) v.clear();
       for (int k = 0; k < ncol; ++k) {

@@ -1,6 +1,6 @@
 // Device executor of the sigma plan (host/plan.h) and the device half of the C
 // ABI.  The FP64 GEMM steps run on gemm_mma_f64.cu; kernels here (FP64):
-//   gemm_skinny_f64   problems of at most 8 rows: a warp per output column
+//   gemm_skinny_f64   problems of at most 8 rows: a warp per two output columns
 //   axpy_segments     one block per target chunk, sources summed in table order
 //   dot_segments      one block per target scalar
 //   unpack_pairs / pack_pairs   SCEP <-> dense external pair matrices
@@ -80,48 +80,53 @@ struct DHead {
   long long off_ab, off_aa, nsf_ab, nsf_aa, nsing, nD, dk0;
 };
 
-// Skinny grouped GEMM (M <= SKINNY_M, B given as N x K): one warp per output
-// column n of a problem computes C[m][n] for every row m as dot products over
-// the segments (lanes along k, fixed-order warp reductions).  Covers the
-// one-row products that would fill 1/64 of a tile of the tiled kernel.  Warp
-// numbers are laid out so that the 8 warps of a block share one problem: the
-// block looks its problem up once, and its warps read the same A rows (L1).
+// Skinny grouped GEMM (M <= SKINNY_M, B given as N x K): one warp per two output columns of a problem computes
+// C[m][n] for every row m as dot products over the segments (lanes along k, fixed-order warp reductions).  Covers the
+// one-row products that would fill 1/64 of a tile of the tiled kernel.  A dot of a few hundred elements is short
+// against what surrounds it: with one column per warp, a binary search for the problem by one thread per block, and a
+// full butterfly per value, 968 products of one integral matrix of 240 externals took 221 us; with two columns on one
+// read of A, 32 probes at a time, the next segment's record loaded ahead and the two columns' sums halved on each other,
+// 123 us (the matrices from HBM: 68).  Every sum as before.
 constexpr int SKINNY_M = 8;
+constexpr int SKINNY_N = 2;  // columns of a warp
 __global__ void __launch_bounds__(256) gemm_skinny_f64(const DGemmProblem* __restrict__ probs, int nprob,
                                                        const DGemmSeg* __restrict__ segs, long long nwarps) {
-  __shared__ int prob_of_block;
-  const long long w0 = (long long)blockIdx.x * 8;  // first warp of the block
-  if (threadIdx.x == 0) {
-    int lo = 0, hi = nprob - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (probs[mid].tile_begin <= w0) lo = mid;
-      else hi = mid - 1;
-    }
-    prob_of_block = lo;
-  }
-  __syncthreads();
-  const long long w = w0 + (threadIdx.x >> 5);
+  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const DGemmProblem P = probs[prob_of_block];
-  const long long n = w - P.tile_begin;
-  if (w >= nwarps || n >= P.N) return;
+  if (w >= nwarps) return;
+  // the problem of this warp (the last with tile_begin <= w), 32 probes at a time
+  int lo = 0, cnt = nprob;
+  while (cnt > 1) {
+    const int step = (cnt + 31) >> 5, off = lane * step;
+    const bool ok = off < cnt && probs[lo + off].tile_begin <= w;
+    const int c = 31 - __clz(__ballot_sync(0xffffffffu, ok));
+    lo += c * step;
+    cnt = min(step, cnt - c * step);
+  }
+  const DGemmProblem P = probs[lo];
+  const long long n0 = SKINNY_N * (w - P.tile_begin), n1 = min(n0 + 1, P.N - 1);  // an odd last one twice
   // each lane keeps sum_q alpha_q (its part of A_m . b_q); one reduction per row at the end
-  double acc[SKINNY_M];
+  double acc[SKINNY_N][SKINNY_M];
 #pragma unroll
-  for (int m = 0; m < SKINNY_M; ++m) acc[m] = 0.0;
+  for (int m = 0; m < SKINNY_M; ++m) acc[0][m] = acc[1][m] = 0.0;
+  DGemmSeg S = {}, next = {};
+  if (P.seg_begin < P.seg_end) next = segs[P.seg_begin];
   for (long long q = P.seg_begin; q < P.seg_end; ++q) {
-    const DGemmSeg S = segs[q];
-    const double* b = S.B + n * S.ldb;
-    // 16-byte loads when both rows start on 16 bytes and K is even
-    const bool vec = ((reinterpret_cast<uintptr_t>(S.A) | reinterpret_cast<uintptr_t>(b)) & 15) == 0 &&
-                     ((S.lda | S.K) & 1) == 0;
-    if (vec && S.K <= 256) {  // the b row in registers once, every row of A against it
-      const double2* b2 = reinterpret_cast<const double2*>(b);
-      const long long h = S.K / 2;
-      double2 y[4];
+    S = next;
+    if (q + 1 < P.seg_end) next = segs[q + 1];
+    const double* b[SKINNY_N] = {S.B + n0 * S.ldb, S.B + n1 * S.ldb};
+    // 16-byte loads when a row of either operand starts on 16 bytes and K is even
+    const bool even = (reinterpret_cast<uintptr_t>(S.A) & 15) == 0 && ((S.lda | S.K) & 1) == 0;
+    const bool vec[SKINNY_N] = {even && (reinterpret_cast<uintptr_t>(b[0]) & 15) == 0,
+                                even && (reinterpret_cast<uintptr_t>(b[1]) & 15) == 0};
+    if (vec[0] && vec[1] && S.K <= 256) {  // the b rows in registers once, every row of A against them
+      const int h = (int)S.K / 2;
+      double2 y[SKINNY_N][4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) y[e] = lane + 32 * e < h ? __ldg(b2 + lane + 32 * e) : make_double2(0.0, 0.0);
+      for (int c = 0; c < SKINNY_N; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          y[c][e] = lane + 32 * e < h ? __ldg(reinterpret_cast<const double2*>(b[c]) + lane + 32 * e) : make_double2(0.0, 0.0);
 #pragma unroll
       for (int m = 0; m < SKINNY_M; ++m) {
         if (m >= P.M) break;
@@ -129,13 +134,16 @@ __global__ void __launch_bounds__(256) gemm_skinny_f64(const DGemmProblem* __res
         double2 x[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) x[e] = lane + 32 * e < h ? __ldg(a2 + lane + 32 * e) : make_double2(0.0, 0.0);
-        double d = 0.0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          d = fma(x[e].x, y[e].x, d);
-          d = fma(x[e].y, y[e].y, d);
+        for (int c = 0; c < SKINNY_N; ++c) {
+          double d = 0.0;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            d = fma(x[e].x, y[c][e].x, d);
+            d = fma(x[e].y, y[c][e].y, d);
+          }
+          acc[c][m] = fma(S.alpha, d, acc[c][m]);
         }
-        acc[m] = fma(S.alpha, d, acc[m]);
       }
       continue;
     }
@@ -143,30 +151,39 @@ __global__ void __launch_bounds__(256) gemm_skinny_f64(const DGemmProblem* __res
     for (int m = 0; m < SKINNY_M; ++m) {
       if (m >= P.M) break;
       const double* a = S.A + m * S.lda;
-      double d = 0.0;
-      if (vec) {
-        const double2* a2 = reinterpret_cast<const double2*>(a);
-        const double2* b2 = reinterpret_cast<const double2*>(b);
-        for (long long k = lane; k < S.K / 2; k += 32) {
-          const double2 x = __ldg(a2 + k), y = __ldg(b2 + k);
-          d = fma(x.x, y.x, d);
-          d = fma(x.y, y.y, d);
+#pragma unroll
+      for (int c = 0; c < SKINNY_N; ++c) {
+        double d = 0.0;
+        if (vec[c]) {
+          const double2* a2 = reinterpret_cast<const double2*>(a);
+          const double2* b2 = reinterpret_cast<const double2*>(b[c]);
+          for (long long k = lane; k < S.K / 2; k += 32) {
+            const double2 x = __ldg(a2 + k), y = __ldg(b2 + k);
+            d = fma(x.x, y.x, d);
+            d = fma(x.y, y.y, d);
+          }
+        } else {
+          for (long long k = lane; k < S.K; k += 32) d = fma(__ldg(a + k), __ldg(b[c] + k), d);
         }
-      } else {
-        for (long long k = lane; k < S.K; k += 32) d = fma(__ldg(a + k), __ldg(b + k), d);
+        acc[c][m] = fma(S.alpha, d, acc[c][m]);
       }
-      acc[m] = fma(S.alpha, d, acc[m]);
     }
   }
+  // lanes 0-15 take the first column's sum, lanes 16-31 the second's
+  const bool second = lane >= 16;
 #pragma unroll
-  for (int m = 0; m < SKINNY_M; ++m)
+  for (int m = 0; m < SKINNY_M; ++m) {
+    if (m >= P.M) break;
+    double v = second ? acc[1][m] : acc[0][m];
+    v += __shfl_xor_sync(0xffffffffu, second ? acc[0][m] : acc[1][m], 16);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], o);
-  if (lane == 0)
-    for (int m = 0; m < SKINNY_M && m < P.M; ++m) {
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const long long n = second ? n0 + 1 : n0;
+    if ((lane & 15) == 0 && n < P.N) {
       double* c = P.C + m * P.ldc + n;
-      *c = (P.beta == 0.0 ? 0.0 : P.beta * *c) + acc[m];
+      *c = (P.beta == 0.0 ? 0.0 : P.beta * *c) + v;
     }
+  }
 }
 
 // The two-external products of a local deck run on local_com.cu over compact squares: per sigma build the pair
@@ -2080,8 +2097,8 @@ struct tci_ctx {
           for (long long q = g.seg_begin; skinny && q < g.seg_end; ++q) skinny = sg[(size_t)q].tA == 0 && sg[(size_t)q].tB == 1;
           if (skinny) {
             DGemmProblem x = g;
-            x.tile_begin = wk;  // first warp (one per output column); a block of 8 warps stays in one problem
-            wk += (g.N + 7) / 8 * 8;
+            x.tile_begin = wk;  // its first warp
+            wk += (g.N + SKINNY_N - 1) / SKINNY_N;
             sk.push_back(x);
           } else {
             reg.push_back(g);

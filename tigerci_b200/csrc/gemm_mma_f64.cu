@@ -7,9 +7,10 @@
 // word read from shared memory feeds eight products instead of four or eight registers' worth of broadcasts, so the
 // pipe, not shared memory or issue slots, sets the rate (the scalar tiled kernels it replaced ran at 10-24 TFLOP/s).
 // Four warps own a 64 x 128 tile, each 64 x 32 of it in 128 accumulator registers, two blocks per SM so that one's
-// copies and barriers run under the other's products; four 16-deep slices in flight by cp.async. Measured on a B200:
-// 592 problems of 256 x 256 x (40 x 256) 31 TFLOP/s, 576 of 173 x 173 x (40 x 173) 23 (6 % of the blocks padding,
-// uneven column shares; 20 with one body for all shapes and predicates for the missing blocks). Against the scalar
+// copies and barriers run under the other's products; four 16-deep slices in flight by cp.async. Tiles of up to 40 rows
+// (48 with odd leading dimensions) leave room for a third block with three slices each: 36 x 28920 x 28920 2.56 -> 2.30
+// ms. Measured on a B200: 592 problems of 256 x 256 x (40 x 256) 31 TFLOP/s, 576 of 173 x 173 x (40 x 173) 24.5 (6 % of
+// the blocks padding, uneven column shares; 20 with one body for all shapes and predicates for the missing blocks). Against the scalar
 // kernels: two-external step at 24 pairs x 173 virtuals 102 -> 35 ms, all-external at 240 virtuals 6.8 -> 5.1 ms. Tried and
 // slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers spill at two blocks per
 // SM), the copies dealt between the products (the loop outgrows the instruction cache: 9-17).
@@ -155,12 +156,13 @@ struct Shape {
   using A = Operand<BM, BK, AM, NT>;
   using B = Operand<(WK > 1 && BM_ == R16 ? BN + 8 : BN), BK, BM_, NT>;  // room for a shifted row
   static constexpr int STAGE = A::SIZE + B::SIZE;  // doubles
-  static constexpr int STG = 4;
+  static constexpr int BLOCKS = WK > 1 ? 1 : MB <= 5 || (MB == 6 && AM == K8 && BM_ == R16) ? 3 : 2;  // per SM
+  static constexpr int STG = BLOCKS == 3 ? 3 : 4;
   static constexpr size_t smem = sizeof(double) * (size_t)STAGE * STG;
 };
 
 template <int MB, int WK, Mode AM, Mode BM_>
-__global__ void __launch_bounds__(threads(WK), WK == 1 ? 2 : 1) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
+__global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS)) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
                                                       const DGemmSeg* __restrict__ segs) {
   using Sh = Shape<MB, WK, AM, BM_>;
   constexpr int NT = Sh::NT, BK = Sh::BK, STG = Sh::STG;
@@ -422,9 +424,12 @@ Place place(const DGemmProblem& g, const Form& f, int bmb, int bnb) {
   // rows and columns of the tiles, in terms of C^T = B^T A^T when the operands change places
   const bool row_k = x.swapped ? f.b_k : f.a_k, col_k = x.swapped ? f.a_k : f.b_k;
   const bool row_even = x.swapped ? f.b_even : f.a_even, col_even = x.swapped ? f.a_even : f.b_even;
-  if (!col_k && !col_even && bnb > NB) bnb = std::min(bnb, 15);  // room for shifted rows
-  x.c = x.swapped ? cut(g.N, g.M, bmb, bnb) : cut(g.M, g.N, bmb, bnb);
   const int modes = !row_k ? (col_k ? 4 : 5) : col_k ? (row_even && col_even ? 0 : 2) : (row_even ? 1 : 3);
+  if (!col_k && !col_even && bnb > NB) bnb = std::min(bnb, 15);  // room for shifted rows
+  // odd leading dimensions, more rows than one tile: six blocks high, three blocks per SM (8-byte copies and uneven
+  // shares leave gaps in the pipe that a third block fills: 173 x 173 x (40 x 173) 10.4 -> 9.7 ms; even ones lose 3-5 %)
+  if (modes == 3 && bnb > NB && (x.swapped ? g.N : g.M) > 64) bmb = std::min(bmb, 6);
+  x.c = x.swapped ? cut(g.N, g.M, bmb, bnb) : cut(g.M, g.N, bmb, bnb);
   x.cls = x.c.mb - 1 + (bnb <= NB ? 8 : 0) + 16 * modes;
   x.work = (bnb <= NB ? (double)x.c.mb * x.c.nb + 4 : (double)x.c.mb * ((x.c.nb + 3) / 4 * 4)) * f.k;
   return x;

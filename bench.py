@@ -742,7 +742,7 @@ def main():
         st = m["stats"]
         if f == "fp64":
             t_dom = (m["prof"]["all-external"] + m["prof"].get("all-external split-k sum", 0.0)) / 1e3
-            kernel, bytes_ = "gemm_panel_f64 split-k (all-external W+/W- product, FP64 FMA)", st["bytes_allext"]
+            kernel, bytes_ = "gemm_mma_f64 split-k (all-external W+/W- product, FP64 matrix instruction)", st["bytes_allext"]
         else:
             t_dom = m["prof"]["all-external"] / 1e3
             kernel = "allext_tf32x3_kernel (tcgen05 kind::tf32, TMA, 3xTF32, FP64 promotion)"

@@ -2,7 +2,7 @@
 // the mixed-precision form (3xTF32 products, FP32 accumulation in TMEM, FP64
 // promotion every few k-steps, FP64 output).
 //
-// Same problem and segment tables as the FP64 SIMT kernel (gemm_tables.h):
+// Same problem and segment tables as the FP64 kernel (gemm_tables.h):
 // every CTA owns one 128 x 64 tile of one problem's C and runs over all of
 // that problem's K segments in table order.  A problem short in M is
 // computed transposed (C^T = B^T A^T, trans_c set) so that its long dimension

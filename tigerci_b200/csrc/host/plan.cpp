@@ -1448,8 +1448,8 @@ void Builder::allext() {
   }
   // FP64 form: Y = U W with the contraction split in S slices (the product has
   // few output rows and a very long k); the slices are summed in order.  S gives
-  // the row-panel kernel (128 columns per block) about eight blocks per SM; the
-  // slices start on multiples of 32 columns of U (16-byte aligned operands).
+  // the FP64 GEMM (tiles of 128 columns) about eight tiles per SM; the slices
+  // start on multiples of 32 columns of U (16-byte aligned operands).
   const i64 offWm = np * np;
   const i64 col_blocks = std::max<i64>(1, (np + 127) / 128);
   const i64 S = std::max<i64>(1, std::min<i64>({16, np / 512, (148 * 8 + col_blocks - 1) / col_blocks}));

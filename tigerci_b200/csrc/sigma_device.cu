@@ -2088,7 +2088,7 @@ struct tci_ctx {
       }
       d.segs = upload(sg, owned, stream);
       {
-        // FP64 form: skinny problems (one-row products) to the warp-per-column kernel, the rest to the matrix
+        // FP64 form: skinny problems (one-row products) to their own kernel, the rest to the matrix
         // instruction
         std::vector<DGemmProblem> sk, reg;
         long long wk = 0;

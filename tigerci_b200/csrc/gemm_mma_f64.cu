@@ -10,9 +10,9 @@
 // copies and barriers run under the other's products; four 16-deep slices in flight by cp.async. Tiles of up to 40 rows
 // (48 with odd leading dimensions) leave room for a third block with three slices each: 36 x 28920 x 28920 2.56 -> 2.30
 // ms. Measured on a B200: 592 problems of 256 x 256 x (40 x 256) 31 TFLOP/s, 576 of 173 x 173 x (40 x 173) 24.5 (6 % of
-// the blocks padding, uneven column shares; 20 with one body for all shapes and predicates for the missing blocks). Against the scalar
-// kernels: two-external step at 24 pairs x 173 virtuals 102 -> 35 ms, all-external at 240 virtuals 6.8 -> 5.1 ms. Tried and
-// slower: four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers spill at two blocks per
+// the blocks padding, uneven column shares; 20 with one body for all shapes and predicates for the missing blocks).
+// Against the scalar kernels: two-external step at 24 pairs x 173 virtuals 102 -> 32 ms, all-external at 240 virtuals
+// 6.8 -> 4.5 ms. Tried and slower: the left-over column blocks of a tile dealt by rows, as a second phase (6-10 %), four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers spill at two blocks per
 // SM), the copies dealt between the products (the loop outgrows the instruction cache: 9-17).
 //
 // A launch of few tiles is bound by the latency of a slice (copy, barrier, products: 1.3 us), one after another: there

@@ -12,8 +12,9 @@
 // ms. Measured on a B200: 592 problems of 256 x 256 x (40 x 256) 31 TFLOP/s, 576 of 173 x 173 x (40 x 173) 24.5 (6 % of
 // the blocks padding, uneven column shares; 20 with one body for all shapes and predicates for the missing blocks).
 // Against the scalar kernels: two-external step at 24 pairs x 173 virtuals 102 -> 32 ms, all-external at 240 virtuals
-// 6.8 -> 4.5 ms. Tried and slower: the left-over column blocks of a tile dealt by rows, as a second phase (6-10 %), four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers spill at two blocks per
-// SM), the copies dealt between the products (the loop outgrows the instruction cache: 9-17).
+// 6.8 -> 4.5 ms. Tried and slower: the left-over column blocks of a tile dealt by rows,
+// as a second phase (6-10 %), four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers
+// spill at two blocks per SM), the copies dealt between the products (the loop outgrows the instruction cache: 9-17).
 //
 // A launch of few tiles is bound by the latency of a slice (copy, barrier, products: 1.3 us), one after another: there
 // eight warps share 64-deep slices of tiles down to 16 x 16. 32 problems of 35 x 35 x (40 x 35): 76 us with four

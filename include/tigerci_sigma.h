@@ -272,6 +272,15 @@ int tci_selftest_gemm_f64(int64_t device, int64_t M, int64_t N, int64_t K, int64
                           int64_t lda, int64_t ldb, int64_t ldc, int64_t a_off, int64_t b_off, int64_t a_step,
                           int64_t b_step, double alpha, double beta, const double* A, int64_t na, const double* B,
                           int64_t nb, double* C);
+/* Its address arithmetic, on the host alone: the asynchronous copies that a
+ * block of tile class cls (0 .. 95: operand modes x work split x row blocks)
+ * makes of one segment's row (which 0) or column (1) operand, nr rows of the
+ * tile x K with leading dimension ld, from element off of an allocation of len
+ * doubles.  out[3] = {copies, copies with an address not aligned to the
+ * instruction's size, copies from outside the allocation or to outside the
+ * shared-memory slice}. */
+int tci_selftest_gemm_f64_copies(int64_t cls, int64_t which, int64_t nr, int64_t K, int64_t ld, int64_t off,
+                                 int64_t len, int64_t* out);
 
 /* ---- A posteriori corrections (calculate_a_posteriori_corrections,
  * tiger_fortran/aposteriori.f90:28-221, called after a one-root SDCI solve,

@@ -64,6 +64,7 @@ EXPORTS = [
     "tci_selftest_bounded_wait",
     "tci_selftest_mma_rate",
     "tci_selftest_gemm_f64",
+    "tci_selftest_gemm_f64_copies",
     "tci_operator_from_records",
     "tci_reference_weight",
     "tci_aposteriori",
@@ -171,6 +172,7 @@ def lib():
         L.tci_selftest_bounded_wait.argtypes = [i64, i64, P, P]
         L.tci_selftest_mma_rate.argtypes = [i64, i64, i64, i64, i64, P]
         L.tci_selftest_gemm_f64.argtypes = [i64] * 14 + [dbl, dbl, P, i64, P, i64, P]
+        L.tci_selftest_gemm_f64_copies.argtypes = [i64] * 7 + [P]
         L.tci_operator_from_records.argtypes = [i64, i64, P, P, i64, P]
         L.tci_reference_weight.argtypes = [P, P, i64, P]
         L.tci_aposteriori.argtypes = [i64, dbl, dbl, P, i64]

@@ -44,6 +44,10 @@ __device__ __forceinline__ void cp_async16(unsigned s, const void* g, int bytes)
 __device__ __forceinline__ void cp_async8(unsigned s, const void* g, int bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(bytes) : "memory");
 }
+struct CpAsync {
+  __device__ __forceinline__ void copy16(unsigned s, const void* g, int bytes) const { cp_async16(s, g, bytes); }
+  __device__ __forceinline__ void copy8(unsigned s, const void* g, int bytes) const { cp_async8(s, g, bytes); }
+};
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -59,15 +63,19 @@ __device__ __forceinline__ void mma884(double& c0, double& c1, double a, double 
 // places.  swz moves bits only, so swz(r0 + r1) = swz(r0) ^ swz(r1) where r0 and r1 share no bits.
 __host__ __device__ constexpr int swz(int r) { return ((r & 3) << 1) | ((r >> 2) & 1); }
 // byte offset of chunk c0 + c1 (no common bits, c1 a constant) of a row with swizzle sw
-__device__ __forceinline__ unsigned chunk(int c0, int c1, int sw) {
+__host__ __device__ __forceinline__ unsigned chunk(int c0, int c1, int sw) {
   return 16u * (unsigned)(((c0 & ~7) + (c1 & ~7)) | ((c0 & 7) ^ (c1 & 7) ^ sw));
 }
 
+// The copies of Operand::issue go to the device (CpAsync) or to a host check of their addresses.
+#pragma nv_diag_suppress 20011, 20014
+
 // How an operand reaches shared memory: rows of the tile with k contiguous by 16-byte (K16) or 8-byte (K8) copies,
 // or with the tile rows contiguous: transposed into the row layout by 8-byte copies (RT8, the row operand), or kept
-// as BK rows of the tile rows, pitch R + 2 (R8, R16, the column operand; reads of two k and eight rows spread over
-// the banks).  16-byte copies want a 16-byte aligned operand with an even leading dimension.
-enum Mode { K16, K8, RT8, R8, R16 };
+// as BK rows of the tile rows, pitch R + 4 (R16, the column operand; reads of two k and eight rows spread over the
+// banks).  K16 wants a 16-byte aligned operand with an even leading dimension; R16 copies the 16-byte words a row lies
+// in, so that a row may start one place into its shared-memory row.
+enum Mode { K16, K8, RT8, R16 };
 
 template <int R, int BK, Mode M, int NT>
 struct Operand {
@@ -83,8 +91,8 @@ struct Operand {
   long long ustep;   // from one pass to the next
   int sh = 0;        // R16: the places this thread's rows are shifted by (0 or 1; PER is even)
   // returns, for R16, the shifts of even (bit 0) and odd (bit 1) k
-  __device__ __forceinline__ int open(const double* X, long long ld, long long row0) {
-    const int x = threadIdx.x % LANES, y = threadIdx.x / LANES;
+  __host__ __device__ __forceinline__ int open(int tid, const double* X, long long ld, long long row0) {
+    const int x = tid % LANES, y = tid / LANES;
     p = X + (KC ? row0 * ld : row0) + (long long)y * ld + (M == K16 || M == R16 ? 2 * x : x);
     ustep = PER * ld;
     if constexpr (M == R16) {
@@ -97,9 +105,11 @@ struct Operand {
     return 0;
   }
   // the slice with min(krem, BK) valid k (zeros past them) into shared memory at s, and on to the next; rows past nr
-  // are left alone: they reach only outputs that are not stored
-  __device__ __forceinline__ void issue(unsigned s, int nr, int krem) {
-    const int x = threadIdx.x % LANES, y = threadIdx.x / LANES;
+  // are left alone: they reach only outputs that are not stored.  A copy of no bytes keeps to its instruction's
+  // alignment and to the operand as well.
+  template <class Copy>
+  __host__ __device__ __forceinline__ void issue(int tid, unsigned s, int nr, int krem, Copy&& to) {
+    const int x = tid % LANES, y = tid / LANES;
     if constexpr (KC) {
       const int k = M == K16 ? 2 * x : x, sw = swz(y);
       const int bytes = max(0, min(M == K16 ? 16 : 8, 8 * (krem - k)));
@@ -109,8 +119,8 @@ struct Operand {
       for (int u = 0; u < U; ++u) {
         const unsigned o = d + 8u * (u * PER * BK) + chunk(k >> 1, 0, sw ^ swz(u * PER));
         if (y + u * PER < nr) {
-          if (M == K16) cp_async16(o, p, bytes);
-          else cp_async8(o, p, bytes);
+          if (M == K16) to.copy16(o, p, bytes);
+          else to.copy8(o, p, bytes);
         }
         p += ustep;
       }
@@ -123,8 +133,8 @@ struct Operand {
         unsigned o;
         if constexpr (KROWS) o = d + 8u * (u * PER * PITCH);
         else o = d + (PER > 1 ? chunk(y >> 1, (u * PER) >> 1, sw) : chunk(0, u >> 1, sw) + 8u * (u & 1));
-        if (M == R16) cp_async16(o, q, n);
-        else cp_async8(o, q, n);
+        if (M == R16) to.copy16(o, q, n);
+        else to.copy8(o, q, n);
       };
       if (krem >= BK) {
 #pragma unroll
@@ -133,7 +143,9 @@ struct Operand {
           p += ustep;
         }
       } else {
-        const double* z = p - y * (ustep / PER);  // about the slice's first k, where nothing is read
+        // where nothing is read: row 0's place at the slice's first k (R16: the 16-byte word that holds it)
+        const double* z = p - y * (ustep / PER) - r;
+        if constexpr (M == R16) z -= (reinterpret_cast<uintptr_t>(z) >> 3) & 1;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const bool ok = y + u * PER < krem;
@@ -225,8 +237,8 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
     const DGemmSeg& S = *reinterpret_cast<const DGemmSeg*>(ring + rs * WORDS);
     krem = (int)S.K;
     alpha = S.alpha;
-    oa.open(tr ? S.B : S.A, tr ? S.ldb : S.lda, m0);
-    flags = 512 * ob.open(tr ? S.A : S.B, tr ? S.lda : S.ldb, n0) + (alpha != 1.0 ? 256 : 0);
+    oa.open(threadIdx.x, tr ? S.B : S.A, tr ? S.ldb : S.lda, m0);
+    flags = 512 * ob.open(threadIdx.x, tr ? S.A : S.B, tr ? S.lda : S.ldb, n0) + (alpha != 1.0 ? 256 : 0);
     // the record RING - 1 ahead takes the place of the one before this, which everyone has left
     const int ahead = sg + RING - 1, pl = rs == 0 ? RING - 1 : rs - 1;
     if (sg > (int)P.seg_begin && ahead < sge && (int)threadIdx.x < WORDS)
@@ -237,8 +249,8 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
   auto produce = [&](int st) {
     if (krem > 0) {
       const unsigned s = sbase + 8u * (unsigned)(st * Sh::STAGE);
-      oa.issue(s, mrows, krem);
-      ob.issue(s + 8u * (unsigned)Sh::A::SIZE, ncols, krem);
+      oa.issue(threadIdx.x, s, mrows, krem, CpAsync());
+      ob.issue(threadIdx.x, s + 8u * (unsigned)Sh::A::SIZE, ncols, krem, CpAsync());
       if (threadIdx.x == 0) {
         meta_alpha[st] = alpha;
         meta_k[st] = min(BK, krem) + flags;
@@ -364,14 +376,13 @@ cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long 
 }
 
 using Go = cudaError_t (*)(const DGemmProblem*, int, const DGemmSeg*, long long, cudaStream_t);
-#define TCI_ROWS(WK, A, B) \
-  go<1, WK, A, B>, go<2, WK, A, B>, go<3, WK, A, B>, go<4, WK, A, B>, go<5, WK, A, B>, go<6, WK, A, B>, go<7, WK, A, B>, \
-      go<8, WK, A, B>
-#define TCI_PAIR(A, B) TCI_ROWS(1, A, B), TCI_ROWS(8, A, B)
-constexpr Go kGo[tci_dmma::CLASSES] = {TCI_PAIR(K16, K16), TCI_PAIR(K16, R16), TCI_PAIR(K8, K8),
-                                       TCI_PAIR(K8, R16),  TCI_PAIR(RT8, K8),  TCI_PAIR(RT8, R16)};
-#undef TCI_PAIR
-#undef TCI_ROWS
+// one F per class
+#define TCI_ROWS(F, WK, A, B) \
+  F<1, WK, A, B>, F<2, WK, A, B>, F<3, WK, A, B>, F<4, WK, A, B>, F<5, WK, A, B>, F<6, WK, A, B>, F<7, WK, A, B>, F<8, WK, A, B>
+#define TCI_PAIR(F, A, B) TCI_ROWS(F, 1, A, B), TCI_ROWS(F, 8, A, B)
+#define TCI_CLASSES(F) \
+  TCI_PAIR(F, K16, K16), TCI_PAIR(F, K16, R16), TCI_PAIR(F, K8, K8), TCI_PAIR(F, K8, R16), TCI_PAIR(F, RT8, K8), TCI_PAIR(F, RT8, R16)
+constexpr Go kGo[tci_dmma::CLASSES] = {TCI_CLASSES(go)};
 
 // Tile counts of a problem of rows x cols: at most bmb row blocks x bnb column blocks.
 struct Cut {
@@ -497,6 +508,52 @@ cudaError_t launch(const Tables& t, const DGemmSeg* segs, cudaStream_t st) {
 }
 
 }  // namespace tci_dmma
+
+// Test entry, host only: the copies that a block of class cls makes of a segment's operand (which 0: the row operand, 1:
+// the column operand): nr rows of the tile x K, leading dimension ld, from element off of an allocation of len doubles.
+// out: {copies, copies with an address not aligned to the instruction's size, copies from outside the allocation or to
+// outside the slice}.
+namespace {
+template <int MB, int WK, Mode AM, Mode BM_>
+void copies_of(int which, int nr, long long K, long long ld, long long off, long long len, int64_t* out) {
+  using Sh = Shape<MB, WK, AM, BM_>;
+  double* const base = reinterpret_cast<double*>((uintptr_t)1 << 40);  // an allocation's alignment; never read
+  struct Count {
+    int64_t* out;
+    uintptr_t lo, hi;
+    unsigned size;
+    void see(unsigned s, const void* g, int bytes, unsigned unit) const {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(g);
+      out[0] += 1;
+      out[1] += a % unit || s % unit;
+      out[2] += a < lo || a + (uintptr_t)std::max(bytes, 1) > hi || s + unit > size || bytes < 0 || bytes > (int)unit;
+    }
+    void copy16(unsigned s, const void* g, int bytes) const { see(s, g, bytes, 16); }
+    void copy8(unsigned s, const void* g, int bytes) const { see(s, g, bytes, 8); }
+  };
+  auto all = [&](auto op) {
+    using Op = decltype(op);
+    const Count c{out, reinterpret_cast<uintptr_t>(base), reinterpret_cast<uintptr_t>(base + len), 8u * (unsigned)Op::SIZE};
+    for (int tid = 0; tid < Sh::NT; ++tid) {
+      Op o;
+      o.open(tid, base + off, ld, 0);
+      for (long long k = K; k > 0; k -= Sh::BK) o.issue(tid, 0, nr, (int)k, c);
+    }
+  };
+  if (which == 0) all(typename Sh::A());
+  else all(typename Sh::B());
+}
+using CopiesOf = void (*)(int, int, long long, long long, long long, long long, int64_t*);
+constexpr CopiesOf kCopies[tci_dmma::CLASSES] = {TCI_CLASSES(copies_of)};
+}  // namespace
+extern "C" int tci_selftest_gemm_f64_copies(int64_t cls, int64_t which, int64_t nr, int64_t K, int64_t ld, int64_t off,
+                                            int64_t len, int64_t* out) {
+  if (!out || cls < 0 || cls >= tci_dmma::CLASSES || which < 0 || which > 1 || nr < 1 || K < 1 || ld < 1 || off < 0)
+    return TCI_ERR_ARG;
+  out[0] = out[1] = out[2] = 0;
+  kCopies[cls]((int)which, (int)nr, K, ld, off, len, out);
+  return TCI_OK;
+}
 
 // Test entry: C (M x N) = beta C + alpha sum_s op(A_s) op(B_s) on host arrays, nseg matrices a_step / b_step apart
 // from element a_off / b_off on.

@@ -4029,7 +4029,7 @@ int tci_ctx_stats(const tci_ctx* ctx, double* out, int64_t len) {
 // device arrays (the dot products of expand_krylov_subspace and the MGS
 // overlaps, tiger_fortran/davidson.f90:478-494, 702-723, for a caller that
 // keeps its Davidson vectors in HBM).  Two-pass reduction in a fixed order:
-// the result does not depend on timing.  Scratch (m * 593 doubles) is owned by
+// the result does not depend on timing.  Scratch (m * 592 doubles) is owned by
 // the context and grows on demand.
 int tci_dots(tci_ctx* ctx, const double* d_A, int64_t lda, int64_t m, const double* d_x, int64_t n, double* d_out,
              void* stream) {
@@ -4066,9 +4066,15 @@ int tci_dots(tci_ctx* ctx, const double* d_A, int64_t lda, int64_t m, const doub
     }
     // about a thousand elements a block, at most the scratch's RBLK blocks a row
     const int nblk = (int)std::min<int64_t>(RBLK, (n + 1023) / 1024);
-    multi_dot_partial<<<dim3((unsigned)nblk, (unsigned)((m + 3) / 4)), RB, 0, run>>>(d_A, lda, (int)m, d_x, n, ctx->dotbuf);
+    constexpr int64_t ROWS = 4 * 65535;  // row groups of a launch: the grid's y
+    for (int64_t k = 0; k < m; k += ROWS) {
+      const int64_t mk = std::min(ROWS, m - k);
+      multi_dot_partial<<<dim3((unsigned)nblk, (unsigned)((mk + 3) / 4)), RB, 0, run>>>(d_A + k * lda, lda, (int)mk, d_x, n,
+                                                                                        ctx->dotbuf + k * nblk);
+      ctx->launch_count += 1;
+    }
     dots_final<<<(unsigned)m, 32, 0, run>>>(ctx->dotbuf, nblk, d_out);
-    ctx->launch_count += 2;
+    ctx->launch_count += 1;
     TCI_CUDA(cudaGetLastError());
     cudaEvent_t done = fork ? ctx->ev0 : ctx->ev_last;
     TCI_CUDA(cudaEventRecord(done, run));

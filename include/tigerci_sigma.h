@@ -281,6 +281,15 @@ int tci_selftest_gemm_f64(int64_t device, int64_t M, int64_t N, int64_t K, int64
  * shared-memory slice}. */
 int tci_selftest_gemm_f64_copies(int64_t cls, int64_t which, int64_t nr, int64_t K, int64_t ld, int64_t off,
                                  int64_t len, int64_t* out);
+/* The two-external products of a local deck on the common virtuals, on host
+ * arrays: one target with m sorted externals dom of n, nsrc sources with ms[s]
+ * externals (sdom: one after the other); A, D: nsrc n x n matrices, D read on
+ * the sources' domains; compact: the rows and columns of A copied together
+ * first.  R[a][b] += sum_s alpha[s] sum_{c in D_s} A_s[a][c] D_s[c][b], a in
+ * dom, b in both domains. */
+int tci_selftest_com(int64_t device, int64_t n, int64_t m, const int64_t* dom, int64_t nsrc, const int64_t* ms,
+                     const int64_t* sdom, const double* alpha, const double* A, const double* D, int64_t compact,
+                     double* R);
 
 /* ---- A posteriori corrections (calculate_a_posteriori_corrections,
  * tiger_fortran/aposteriori.f90:28-221, called after a one-root SDCI solve,

@@ -16,6 +16,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "../../include/tigerci_sigma.h"
 #include "local_com.h"
 
 namespace {
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(NT, 2) com_products(const Task* __restrict__ t
   extern __shared__ __align__(128) double sm[];
   __shared__ double s_alpha[SLOTS];
   __shared__ int s_cnt[SLOTS], s_nsl[SLOTS], s_ct[SLOTS][COLS];
-  double* Y = sm + STG * STAGE;  // [position in the target's domain][row]
+  double* Y = sm + STG * STAGE;  // [position in the target's domain - c0][row]
   const Task T = tasks[blockIdx.x];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
   // four row shares of the tile, rotated over the schedulers, two column shares
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(NT, 2) com_products(const Task* __restrict__ t
       s_cnt[pslot] = J.cnt;
       s_nsl[pslot] = (J.m + BK - 1) / BK;
     }
-    if (tid < J.cnt) s_ct[pslot][tid] = nct;
+    if (tid < J.cnt) s_ct[pslot][tid] = nct - T.c0;
     if (pj + 1 < T.job1) N = jobs[pj + 1];
   };
   if (pj < T.job1) open();
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(NT, 2) com_products(const Task* __restrict__ t
   __syncthreads();
   for (int r = warp; r < T.rows; r += NT / 32) {
     double* row = T.R + (long long)T.dom[T.r0 + r] * ld;
-    for (int c = lane; c < T.m; c += 32) row[T.dom[c]] += Y[c * YP + r];
+    for (int c = lane; c < T.m; c += 32) row[T.dom[T.c0 + c]] += Y[c * YP + r];
   }
 }
 
@@ -212,14 +213,47 @@ cudaError_t go(const Task* tasks, int ntasks, int mmax, const Job* jobs, long lo
 
 namespace tci_com {
 
-// 64 and 32 rows leave room for two blocks per SM (113 KB each); larger domains take what one block can hold.
-int task_class(int m) {
-  if (m <= 126) return 0;
-  if (m <= 280) return 1;
-  if (m <= 1200) return 2;
-  return m <= 2100 ? 3 : -1;
+// 64 and 32 rows leave room for two blocks per SM (113 KB each); larger domains take what one block can hold, and above
+// that their columns are cut in even windows of the 16-row class.
+static int task_class(int m) { return m <= 126 ? 0 : m <= 280 ? 1 : m <= 1200 ? 2 : 3; }
+constexpr int MAX_COLS = 2100, WINDOW = 1200;
+
+void HostPlan::add(double* R, const int* dom, int m, const std::vector<Term>& terms) {
+  const int nwin = m <= MAX_COLS ? 1 : (m + WINDOW - 1) / WINDOW;
+  for (int w = 0; w < nwin; ++w) {
+    const int c0 = (int)((long long)m * w / nwin), c1 = (int)((long long)m * (w + 1) / nwin);
+    const int cls = task_class(c1 - c0), job0 = (int)jobs.size();
+    double work = 0;
+    for (const Term& x : terms) {
+      // the term's columns in the window, COLS at a time
+      const int f0 = (int)(std::lower_bound(x.host_ct, x.host_ct + x.job.cnt, c0) - x.host_ct);
+      const int n = (int)(std::lower_bound(x.host_ct + f0, x.host_ct + x.job.cnt, c1) - x.host_ct) - f0;
+      const int parts = (n + COLS - 1) / COLS;
+      for (int q = 0; q < parts; ++q) {
+        const int f = f0 + (int)((long long)n * q / parts), e = f0 + (int)((long long)n * (q + 1) / parts);
+        Job j = x.job;
+        j.cs += f;
+        j.ct += f;
+        j.cnt = e - f;
+        jobs.push_back(j);
+        work += (double)((j.m + 15) / 16) * (double)(8 + j.cnt);
+      }
+    }
+    if (job0 == (int)jobs.size()) continue;
+    const int rows = 64 >> cls, nt = (m + rows - 1) / rows;  // even row tiles
+    for (int t = 0; t < nt; ++t) {
+      const int f = (int)((long long)m * t / nt), e = (int)((long long)m * (t + 1) / nt);
+      tasks[cls].push_back(HostTask{work, Task{R, dom, c1 - c0, f, e - f, job0, (int)jobs.size(), c0}});
+    }
+  }
 }
-int class_rows(int cls) { return 64 >> cls; }
+
+std::vector<Task> HostPlan::sorted(int cls) {
+  std::stable_sort(tasks[cls].begin(), tasks[cls].end(), [](const HostTask& x, const HostTask& y) { return x.work > y.work; });
+  std::vector<Task> v;
+  for (const auto& x : tasks[cls]) v.push_back(x.t);
+  return v;
+}
 
 cudaError_t launch(const Tables& t, long long ld, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
@@ -231,3 +265,84 @@ cudaError_t launch(const Tables& t, long long ld, cudaStream_t st) {
 }
 
 }  // namespace tci_com
+
+// Test entry on host arrays: one target with m externals dom of n, nsrc sources with ms[s] externals (sdom, one after the
+// other), A (nsrc x n x n) and D (nsrc x n x n, read on the sources' domains): R (n x n) += the terms' products on the
+// common columns.
+extern "C" int tci_selftest_com(int64_t device, int64_t n, int64_t m, const int64_t* dom, int64_t nsrc, const int64_t* ms,
+                                const int64_t* sdom, const double* alpha, const double* A, const double* D, int64_t compact,
+                                double* R) {
+  if (n < 1 || m < 1 || m > n || nsrc < 1 || !dom || !ms || !sdom || !alpha || !A || !D || !R) return TCI_ERR_ARG;
+  std::vector<void*> owned;
+  int rc = TCI_OK;
+  auto ok = [&](cudaError_t e) {
+    if (e != cudaSuccess && rc == TCI_OK) rc = TCI_ERR_CUDA;
+    return rc == TCI_OK;
+  };
+  auto up = [&](const auto& v) {
+    using V = typename std::decay<decltype(v[0])>::type;
+    void* p = nullptr;
+    if (ok(cudaMalloc(&p, sizeof(V) * std::max<size_t>(1, v.size())))) {
+      owned.push_back(p);
+      if (!v.empty()) ok(cudaMemcpy(p, v.data(), sizeof(V) * v.size(), cudaMemcpyHostToDevice));
+    }
+    return static_cast<V*>(p);
+  };
+  try {
+    const auto sorted_in = [&](const int64_t* d, int64_t c) {
+      for (int64_t i = 0; i < c; ++i)
+        if (d[i] < 0 || d[i] >= n || (i > 0 && d[i] <= d[i - 1])) return false;
+      return true;
+    };
+    if (!sorted_in(dom, m)) return TCI_ERR_ARG;
+    for (int64_t s = 0, o = 0; s < nsrc; o += ms[s++])
+      if (ms[s] < 1 || ms[s] > n || !sorted_in(sdom + o, ms[s])) return TCI_ERR_ARG;
+    ok(cudaSetDevice((int)device));
+    std::vector<std::vector<int>> cts;
+    std::vector<tci_com::Term> terms;
+    const int* d_dom = up(std::vector<int>(dom, dom + m));
+    for (int64_t s = 0, o = 0; s < nsrc && rc == TCI_OK; o += ms[s++]) {
+      const int64_t k = ms[s], p = k + (k & 1), *sd = sdom + o;
+      std::vector<int> cs, ct;
+      for (int64_t x = 0; x < k; ++x) {
+        const int64_t* y = std::lower_bound(dom, dom + m, sd[x]);
+        if (y < dom + m && *y == sd[x]) cs.push_back((int)x), ct.push_back((int)(y - dom));
+      }
+      if (cs.empty()) continue;
+      std::vector<double> sq((size_t)(k * p)), a;
+      const double *As = A + s * n * n, *Ds = D + s * n * n;
+      for (int64_t r = 0; r < k; ++r)
+        for (int64_t c = 0; c < k; ++c) sq[(size_t)(r * p + c)] = Ds[sd[r] * n + sd[c]];
+      if (compact) {
+        a.resize((size_t)(m * p));
+        for (int64_t r = 0; r < m; ++r)
+          for (int64_t c = 0; c < k; ++c) a[(size_t)(r * p + c)] = As[dom[r] * n + sd[c]];
+      } else {
+        a.assign(As, As + n * n);
+      }
+      cts.push_back(ct);
+      const double *da = up(a), *db = up(sq);
+      const int *dd = up(std::vector<int>(sd, sd + k)), *dcs = up(cs), *dct = up(ct);
+      terms.push_back({Job{da, db, dd, dcs, dct, (int)k, (int)cs.size(), (int)p, (int)p, alpha[s], compact ? 1 : 0, 0}, nullptr});
+    }
+    for (size_t i = 0; i < terms.size(); ++i) terms[i].host_ct = cts[i].data();
+    double* d_R = up(std::vector<double>(R, R + n * n));
+    tci_com::HostPlan plan;
+    plan.add(d_R, d_dom, (int)m, terms);
+    tci_com::Tables t;
+    for (int c = 0; c < tci_com::CLASSES; ++c) {
+      const std::vector<Task> v = plan.sorted(c);
+      for (const Task& x : v) t.mmax[c] = std::max(t.mmax[c], x.m);
+      t.tasks[c] = up(v);
+      t.ntasks[c] = (int)v.size();
+    }
+    t.jobs = up(plan.jobs);
+    if (rc == TCI_OK) ok(tci_com::launch(t, n, 0));
+    ok(cudaDeviceSynchronize());
+    if (rc == TCI_OK) ok(cudaMemcpy(R, d_R, sizeof(double) * (size_t)(n * n), cudaMemcpyDeviceToHost));
+  } catch (...) {
+    rc = TCI_ERR_INTERNAL;
+  }
+  for (void* p : owned) cudaFree(p);
+  return rc;
+}

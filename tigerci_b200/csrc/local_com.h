@@ -19,16 +19,34 @@ struct Job {
   double alpha;
   int compact, pad;
 };
-// Rows [r0, r0 + rows) of the target's domain, added into its padded pair matrix R at the end.
+// Rows [r0, r0 + rows) and columns [c0, c0 + m) of the target's domain, added into its padded pair matrix R at the end;
+// the jobs' ct lie in the columns.
 struct Task {
   double* R;
   const int* dom;
-  int m, r0, rows, job0, job1, pad;
+  int m, r0, rows, job0, job1, c0;
 };
-// Row tiles by domain size: the tile's sums (domain size x rows) live in shared memory.
+// Row tiles by number of columns: the tile's sums (columns x rows) live in shared memory.
 constexpr int CLASSES = 4;
-int task_class(int m);       // -1: larger than any class holds
-int class_rows(int cls);
+// One term of a target: the operands as in Job, all its common columns, their positions in the target's domain also on
+// the host (ascending).
+struct Term {
+  Job job;
+  const int* host_ct;
+};
+// The tasks and jobs of a launch.
+struct HostPlan {
+  struct HostTask {
+    double work;
+    Task t;
+  };
+  std::vector<Job> jobs;
+  std::vector<HostTask> tasks[CLASSES];
+  // one target: its padded pair matrix, domain (device) and terms
+  void add(double* R, const int* dom, int m, const std::vector<Term>& terms);
+  // a class's tasks, the longest first
+  std::vector<Task> sorted(int cls);
+};
 struct Tables {
   Task* tasks[CLASSES] = {};
   int ntasks[CLASSES] = {}, mmax[CLASSES] = {};

@@ -1620,48 +1620,26 @@ struct tci_ctx {
                (int)pitch_of(mh(h))};
       if (src_used[(size_t)dk]) gsq.push_back(q);
     }
-    // tasks: even row tiles of each target, the longest first; jobs: each term's common columns, COLS at a time
-    std::vector<tci_com::Job> cj;
-    struct HostTask {
-      double work;
-      tci_com::Task t;
-    };
-    std::vector<HostTask> ct[tci_com::CLASSES];
+    tci_com::HostPlan hp;
     for (const auto& p : probs) {
-      const int cls = tci_com::task_class((int)p.m);
-      if (cls < 0) throw Error(TCI_ERR_INPUT, "pair domain too large for the two-external step");
-      const int job0 = (int)cj.size();
-      double work = 0;
+      std::vector<tci_com::Term> terms;
       for (const auto& x : p.segs) {
         const i64 ms = mh(x.hs);
         const double* ac = abuf ? abuf + apos.at(std::make_tuple(x.A, p.head, x.hs)) : nullptr;
-        const i64 parts = (x.ncol + tci_com::COLS - 1) / tci_com::COLS;
-        for (i64 q = 0; q < parts; ++q) {
-          const i64 f = x.ncol * q / parts, e = x.ncol * (q + 1) / parts;
-          cj.push_back(tci_com::Job{ac ? ac : x.A, dsq + sq_off[(size_t)x.dks], ddom + ls.dh_off[(size_t)x.hs],
-                                    dcs + x.col_off + f, dct + x.col_off + f, (int)ms, (int)(e - f), (int)pitch_of(ms),
-                                    (int)pitch_of(ms), x.alpha, ac ? 1 : 0, 0});
-          work += (double)((ms + 15) / 16) * (double)(8 + (e - f));
-        }
+        terms.push_back({tci_com::Job{ac ? ac : x.A, dsq + sq_off[(size_t)x.dks], ddom + ls.dh_off[(size_t)x.hs],
+                                      dcs + x.col_off, dct + x.col_off, (int)ms, (int)x.ncol, (int)pitch_of(ms),
+                                      (int)pitch_of(ms), x.alpha, ac ? 1 : 0, 0},
+                         cpos_t.data() + x.col_off});
       }
-      const int rows = tci_com::class_rows(cls), nt = ((int)p.m + rows - 1) / rows;
-      for (int t = 0; t < nt; ++t) {
-        const int f = (int)(p.m * t / nt), e = (int)(p.m * (t + 1) / nt);
-        ct[cls].push_back(HostTask{work, tci_com::Task{buf[BUF_R] + p.dk * n2, ddom + ls.dh_off[(size_t)p.head], (int)p.m, f,
-                                                       e - f, job0, (int)cj.size(), 0}});
-      }
+      hp.add(buf[BUF_R] + p.dk * n2, ddom + ls.dh_off[(size_t)p.head], (int)p.m, terms);
     }
     for (int c = 0; c < tci_com::CLASSES; ++c) {
-      std::stable_sort(ct[c].begin(), ct[c].end(), [](const HostTask& x, const HostTask& y) { return x.work > y.work; });
-      std::vector<tci_com::Task> v;
-      for (const auto& x : ct[c]) {
-        v.push_back(x.t);
-        d.com.mmax[c] = std::max(d.com.mmax[c], x.t.m);
-      }
+      const std::vector<tci_com::Task> v = hp.sorted(c);
+      for (const auto& x : v) d.com.mmax[c] = std::max(d.com.mmax[c], x.m);
       d.com.tasks[c] = upload(v, owned, stream);
       d.com.ntasks[c] = (int)v.size();
     }
-    d.com.jobs = upload(cj, owned, stream);
+    d.com.jobs = upload(hp.jobs, owned, stream);
     d.com_pack = upload(jobs, owned, stream);
     d.com_njobs = (long long)jobs.size();
     d.com_gather = upload(gsq, owned, stream);

@@ -290,6 +290,13 @@ int tci_selftest_gemm_f64_copies(int64_t cls, int64_t which, int64_t nr, int64_t
 int tci_selftest_com(int64_t device, int64_t n, int64_t m, const int64_t* dom, int64_t nsrc, const int64_t* ms,
                      const int64_t* sdom, const double* alpha, const double* A, const double* D, int64_t compact,
                      double* R);
+/* The tables of the integral form of the pair-domain all-external term, on the
+ * host alone: nblocks singlet-coupled blocks with the domains dom_idx[dom_off
+ * .. dom_off + dom_len), for sms multiprocessors.  out[5] = {their indexes fit
+ * 32 bits (0: the rest is 0 and nothing is built), copies of sigma, tasks,
+ * jobs, entries of the columns' list}. */
+int tci_selftest_integral_plan(int64_t num_external, int64_t nblocks, const int64_t* dom_off, const int64_t* dom_len,
+                               const int64_t* dom_idx, int64_t ndom, int64_t sms, int64_t* out);
 
 /* ---- A posteriori corrections (calculate_a_posteriori_corrections,
  * tiger_fortran/aposteriori.f90:28-221, called after a one-root SDCI solve,
@@ -344,8 +351,9 @@ int tci_local_allext_records(const tci_deck* deck, int64_t* out, int64_t cap, in
  * where the device has room for X = Lpk Lpk^T and the W tiles), 1 Cholesky,
  * 2 dense (TCI_ERR_INPUT in FP64 or with a triplet-coupled aa block,
  * TCI_ERR_MEMORY without the room), 3 integrals on the domains (TCI_ERR_INPUT
- * in the mixed precision or with a triplet-coupled aa block, TCI_ERR_MEMORY
- * without the room). */
+ * in the mixed precision, with a triplet-coupled aa block, with more than 2000
+ * externals or with sum n^2 >= 2^31 over the blocks, TCI_ERR_MEMORY without
+ * the room). */
 typedef struct tci_local tci_local;
 int tci_local_create(int64_t num_internal, int64_t num_external, const double* chol, int64_t nchol, int64_t n_heads,
                      const int64_t* heads, const int64_t* dom_idx, int64_t total_len, int64_t device,

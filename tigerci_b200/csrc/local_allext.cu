@@ -52,6 +52,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <string>
 #include <unordered_map>
@@ -492,9 +493,12 @@ struct tci_local {
     dense_ready = true;
   }
 
-  // Integral form (FP64): the kernel's tables, host side.
-  void plan_integral(const std::vector<long long>& dom, tci_lint::Plan& P) const {
+  // Integral form (FP64): the kernel's tables, host side; false where their indexes do not reach.
+  bool plan_integral(const std::vector<long long>& dom, int sms, tci_lint::Plan& P) const {
     std::vector<int> di, dp;
+    double len = 0;
+    for (const auto& H : heads) len += (double)H.n;
+    if (len > (double)std::numeric_limits<int>::max()) return false;
     for (const auto& H : heads) {
       dp.push_back((int)di.size());
       for (long long a = 0; a < H.n; ++a) di.push_back((int)dom[(size_t)(H.dom_off + a)]);
@@ -503,7 +507,9 @@ struct tci_local {
     for (const auto& B : blocks)
       bl.push_back(tci_lint::Block{B.ab ? B.off_ab + B.k * (B.n * (B.n - 1) / 2) : -1, B.aa ? B.off_aa + B.k * B.n : -1, B.p,
                                    (int)B.n, dp[(size_t)B.head], (int)B.head, 0});
-    tci_lint::make_plan((int)nvirt, (int)heads.size(), di, std::move(bl), (int)tci_dev::device_sms(), P);
+    if (!tci_lint::fits(bl)) return false;
+    tci_lint::make_plan((int)nvirt, (int)heads.size(), di, std::move(bl), sms, P);
+    return true;
   }
   // Its set-up from the virtual-virtual Cholesky rows lpk: X by row panels of its lower triangle on the FP64 GEMM,
   // mirrored, and the tables.
@@ -797,7 +803,10 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       if (want_form == 3 && !room) throw Error(TCI_ERR_MEMORY, "not enough device memory for the integral all-external form");
       integral = want_form == 3 || (room && (budget >= 16e9 || xb + cb <= budget) &&
                                     3.0 * L->flops >= (double)L->npv * (double)L->npv * (double)nchol);
-      if (integral) L->plan_integral(dom, iplan);
+      if (integral && !L->plan_integral(dom, (int)tci_dev::device_sms(), iplan)) {
+        if (want_form == 3) throw Error(TCI_ERR_INPUT, "too many blocks for the integral all-external form");
+        integral = false;
+      }
       if (want_form != 3 && 1.5 * iplan.flops > L->flops) integral = false;
     }
     const bool chol_form = want_form != 2 && !integral;

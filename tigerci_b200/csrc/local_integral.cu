@@ -17,9 +17,11 @@
 // 11 at 150 pairs of 20-150 of 300 externals), and n^2 sum n_h^2 products replace the Cholesky form's 4 nchol sum n_h^3.
 // Bound by the copies (9.9 ms alone) and the products of half-filled tiles (11.4 alone) together.  Every sum in a fixed order.
 #include <algorithm>
+#include <limits>
 #include <mutex>
 #include <type_traits>
 
+#include "../../include/tigerci_sigma.h"
 #include "local_integral.h"
 
 namespace {
@@ -270,6 +272,12 @@ __global__ void __launch_bounds__(256) mirror_lower(double* __restrict__ X, long
 
 namespace tci_lint {
 
+bool fits(const std::vector<Block>& blocks) {
+  double entries = 0;  // of jcol; the other lists are no longer
+  for (const Block& b : blocks) entries += (double)b.n * (double)b.n;
+  return entries <= (double)std::numeric_limits<int>::max();
+}
+
 void make_plan(int nv, int nheads, const std::vector<int>& dom, std::vector<Block> blocks, int sms, Plan& P) {
   P.nv = nv;
   P.dom = dom;
@@ -365,3 +373,36 @@ cudaError_t launch(const Device& d, const double* X, int64_t npv, const double* 
 }
 
 }  // namespace tci_lint
+
+// Test entry, host only: the plan of nblocks singlet-coupled blocks with the domains dom_idx[dom_off .. + dom_len) for sms
+// multiprocessors. out: {the lists fit (0: nothing else is set), parts, tasks, jobs, entries of the columns' list}.
+extern "C" int tci_selftest_integral_plan(int64_t num_external, int64_t nblocks, const int64_t* dom_off, const int64_t* dom_len,
+                                          const int64_t* dom_idx, int64_t ndom, int64_t sms, int64_t* out) {
+  if (num_external < 1 || num_external > tci_lint::MAX_NV || nblocks < 1 || ndom < 1 || sms < 1 || !dom_off || !dom_len ||
+      !dom_idx || !out)
+    return TCI_ERR_ARG;
+  try {
+    std::vector<int> dom;
+    for (int64_t i = 0; i < ndom; ++i) {
+      if (dom_idx[i] < 0 || dom_idx[i] >= num_external) return TCI_ERR_ARG;
+      dom.push_back((int)dom_idx[i]);
+    }
+    std::vector<Block> bl;
+    for (int64_t b = 0; b < nblocks; ++b) {
+      if (dom_off[b] < 0 || dom_len[b] < 1 || dom_off[b] + dom_len[b] > ndom) return TCI_ERR_ARG;
+      bl.push_back(Block{0, 0, 1.0, (int)dom_len[b], (int)dom_off[b], (int)b, 0});
+    }
+    for (int k = 0; k < 5; ++k) out[k] = 0;
+    if (!tci_lint::fits(bl)) return TCI_OK;
+    tci_lint::Plan P;
+    tci_lint::make_plan((int)num_external, (int)nblocks, dom, std::move(bl), (int)sms, P);
+    out[0] = 1;
+    out[1] = P.parts;
+    out[2] = (int64_t)P.tasks.size();
+    out[3] = (int64_t)P.jobs.size();
+    out[4] = (int64_t)P.jcol.size();
+    return TCI_OK;
+  } catch (...) {
+    return TCI_ERR_INTERNAL;
+  }
+}

@@ -44,7 +44,9 @@ struct Device {
 // Row pitch of the padded pair matrices.
 inline int64_t pitch(int64_t nv) { return (nv + 15) / 16 * 16; }
 constexpr int64_t MAX_NV = 2000;
-// sms: multiprocessors to fill.
+// The tables index their lists (the longest holds n_h^2 entries per block) in 32 bits: do these blocks' fit?
+bool fits(const std::vector<Block>& blocks);
+// sms: multiprocessors to fill. The blocks fit.
 void make_plan(int nv, int nheads, const std::vector<int>& dom, std::vector<Block> blocks, int sms, Plan& out);
 // X (npv x npv) from its lower triangle.
 cudaError_t mirror(double* X, int64_t npv, cudaStream_t st);

@@ -345,16 +345,23 @@ int tci_local_allext_records(const tci_deck* deck, int64_t* out, int64_t cap, in
  * whichever a timed run at set-up finds faster; in FP64 from the packed
  * integrals over the domains where the device has room for them and they pay
  * (8 npv^2 bytes, npv = num_external (num_external + 1) / 2).  options: [0] precision
- * (TCI_PRECISION_*), [1] device bytes for the per-chunk buffers (default
- * 16e9), [2] promotion block, [3] 0 to skip the set-up autotuning of chunk
+ * (TCI_PRECISION_*), [1] device bytes for the per-chunk buffers (0: the
+ * default, 16e9), [2] promotion block, [3] 0 to skip the set-up autotuning of chunk
  * size and tile shape, [4] form: 0 the faster (default; the dense form only
  * where the device has room for X = Lpk Lpk^T and the W tiles), 1 Cholesky,
  * 2 dense (TCI_ERR_INPUT in FP64 or with a triplet-coupled aa block,
  * TCI_ERR_MEMORY without the room), 3 integrals on the domains (TCI_ERR_INPUT
  * in the mixed precision, with a triplet-coupled aa block, with more than 2000
  * externals or with sum n^2 >= 2^31 over the blocks, TCI_ERR_MEMORY without
- * the room). */
+ * the room), [5] device bytes that form 0 may give to the integrals of form 3
+ * and their padded pair matrices, which stay for the operator's life (0: as
+ * [1] if that is given and not its default, else 0.6 of the free memory).
+ * Form 3 multiplies zeros outside the domains: an infinity or NaN in chol
+ * reaches every block, in form 1 the blocks whose domains hold its externals. */
 typedef struct tci_local tci_local;
+/* The largest single device allocation, in bytes, that tci_local_create may
+ * make in the calling thread (0: no limit): a full device for tests. */
+int tci_selftest_local_alloc_limit(int64_t bytes);
 int tci_local_create(int64_t num_internal, int64_t num_external, const double* chol, int64_t nchol, int64_t n_heads,
                      const int64_t* heads, const int64_t* dom_idx, int64_t total_len, int64_t device,
                      const int64_t* options, int64_t n_options, tci_local** out);

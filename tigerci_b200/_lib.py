@@ -67,6 +67,7 @@ EXPORTS = [
     "tci_selftest_gemm_f64_copies",
     "tci_selftest_com",
     "tci_selftest_integral_plan",
+    "tci_selftest_local_alloc_limit",
     "tci_operator_from_records",
     "tci_reference_weight",
     "tci_aposteriori",
@@ -176,6 +177,7 @@ def lib():
         L.tci_selftest_gemm_f64.argtypes = [i64] * 14 + [dbl, dbl, P, i64, P, i64, P]
         L.tci_selftest_gemm_f64_copies.argtypes = [i64] * 7 + [P]
         L.tci_selftest_integral_plan.argtypes = [i64, i64, P, P, P, i64, i64, P]
+        L.tci_selftest_local_alloc_limit.argtypes = [i64]
         L.tci_selftest_com.argtypes = [i64, i64, i64, P, i64, P, P, P, P, P, i64, P]
         L.tci_operator_from_records.argtypes = [i64, i64, P, P, i64, P]
         L.tci_reference_weight.argtypes = [P, P, i64, P]

@@ -267,6 +267,12 @@ __global__ void add_into(double* __restrict__ dst, const double* __restrict__ sr
     dst[i] += src[i];
 }
 
+constexpr double DEFAULT_BUDGET = 16e9;  // device bytes of the per-chunk buffers
+
+// the largest single allocation of an operator's set-up in this thread (0: no limit), for tests of a full device
+thread_local int64_t t_alloc_limit = 0;
+bool within_limit(size_t bytes) { return t_alloc_limit <= 0 || bytes <= (size_t)t_alloc_limit; }
+
 struct GemmLaunch {
   tci_dmma::Tables t;
   DGemmSeg* segs = nullptr;
@@ -340,7 +346,7 @@ struct tci_local {
   T* upload(const std::vector<T>& v) {
     if (v.empty()) return nullptr;
     T* d = nullptr;
-    if (cudaMalloc(&d, v.size() * sizeof(T)) != cudaSuccess) {
+    if (!within_limit(v.size() * sizeof(T)) || cudaMalloc(&d, v.size() * sizeof(T)) != cudaSuccess) {
       cudaGetLastError();
       throw Error(TCI_ERR_MEMORY, "device allocation failed (local all-external tables)");
     }
@@ -367,7 +373,7 @@ struct tci_local {
   float* alloc_f(size_t n) { return reinterpret_cast<float*>(alloc((n + 1) / 2)); }
   double* alloc(size_t n) {
     double* p = nullptr;
-    if (cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(double)) != cudaSuccess) {
+    if (!within_limit(n * sizeof(double)) || cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       throw Error(TCI_ERR_MEMORY, "device allocation failed (local all-external buffers)");
     }
@@ -491,6 +497,20 @@ struct tci_local {
     dense_flops = 2.0 * (double)np_d * (double)np_d * (double)nsing_d + 2.0 * (double)nm_d * (double)nm_d * (double)ntrip_d;
     dense_bytes = 4.0 * ((double)tci_tc_host::w32_floats(np_d) + (nm_d > 0 ? (double)tci_tc_host::w32_floats(nm_d) : 0.0));
     dense_ready = true;
+  }
+
+  // frees every allocation made after the first `mark`
+  void release_after(size_t mark) {
+    LCUDA(cudaStreamSynchronize(stream));
+    for (size_t i = mark; i < owned.size(); ++i) {
+      auto sz = sizes.find(owned[i]);
+      if (sz != sizes.end()) {
+        dev_bytes -= sz->second;
+        sizes.erase(sz);
+      }
+      LCUDA(cudaFree(owned[i]));
+    }
+    owned.resize(mark);
   }
 
   // Integral form (FP64): the kernel's tables, host side; false where their indexes do not reach.
@@ -687,6 +707,11 @@ struct tci_local {
 
 extern "C" {
 
+int tci_selftest_local_alloc_limit(int64_t bytes) {
+  t_alloc_limit = bytes;
+  return TCI_OK;
+}
+
 int tci_local_create(int64_t num_internal, int64_t num_external, const double* chol, int64_t nchol, int64_t n_heads,
                      const int64_t* heads, const int64_t* dom_idx, int64_t total_len, int64_t device,
                      const int64_t* options, int64_t n_options, tci_local** out) {
@@ -701,7 +726,7 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
     L->nchol = nchol;
     L->total = total_len;
     L->precision = (options && n_options > 0) ? options[0] : 0;
-    const double budget = (options && n_options > 1 && options[1] > 0) ? (double)options[1] : 16e9;
+    const double budget = (options && n_options > 1 && options[1] > 0) ? (double)options[1] : DEFAULT_BUDGET;
     if (options && n_options > 2 && options[2] > 0) L->kblock = options[2];
     const bool tune = !(options && n_options > 3 && options[3] == 0);
     const int64_t want_form = (options && n_options > 4) ? options[4] : 0;  // 0 faster, 1 Cholesky, 2 dense, 3 integral
@@ -784,9 +809,10 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       if (B.aa && B.p < 0.0) dense = false;
     if (want_form == 2 && !dense)
       throw Error(TCI_ERR_INPUT, "the dense all-external form needs the mixed precision and singlet-coupled aa blocks");
-    // FP64: the integrals on the domains where the device has room for X and it costs no more to set up than the
-    // Cholesky form's timed runs (X takes npv^2 nchol flops, three runs 3 x flops; at 150 pairs of 20-150 of 300
-    // externals the application goes 81 -> 11 ms), a caller's chunk budget below the default bounding X too
+    // FP64: the integrals on the domains where the device has room for X, within the bytes the caller allows, and it
+    // costs no more to set up than the Cholesky form's timed runs (X takes npv^2 nchol flops, three runs 3 x flops; at 150
+    // pairs of 20-150 of 300 externals the application goes 81 -> 13.6 ms). X stays for the operator's life, so by default it
+    // takes at most 0.6 of what is free: room for the vectors and the next operator.
     bool integral = L->precision == 0 && want_form != 1 && want_form != 2 && num_external <= tci_lint::MAX_NV;
     for (const auto& B : L->blocks)
       if (B.aa && B.p < 0.0) integral = false;
@@ -801,7 +827,10 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       LCUDA(cudaMemGetInfo(&free_b, &total_b));
       const bool room = need < (want_form == 3 ? 1.0 : 0.6) * (double)free_b;
       if (want_form == 3 && !room) throw Error(TCI_ERR_MEMORY, "not enough device memory for the integral all-external form");
-      integral = want_form == 3 || (room && (budget >= 16e9 || xb + cb <= budget) &&
+      const double allowed = (options && n_options > 5 && options[5] > 0) ? (double)options[5]
+                             : budget != DEFAULT_BUDGET                   ? budget
+                                                                          : (double)free_b;
+      integral = want_form == 3 || (room && xb + cb <= allowed &&
                                     3.0 * L->flops >= (double)L->npv * (double)L->npv * (double)nchol);
       if (integral && !L->plan_integral(dom, (int)tci_dev::device_sms(), iplan)) {
         if (want_form == 3) throw Error(TCI_ERR_INPUT, "too many blocks for the integral all-external form");
@@ -809,7 +838,7 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       }
       if (want_form != 3 && 1.5 * iplan.flops > L->flops) integral = false;
     }
-    const bool chol_form = want_form != 2 && !integral;
+    bool chol_form = want_form != 2 && !integral;
     if (dense) {
       // device bytes it needs at set-up (X, the split Cholesky rows, the W tiles, U and Y), with the
       // Cholesky form's buffers when both are timed, against what the device has free
@@ -842,7 +871,20 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       double* tmp = L->alloc(lvv.size());
       LCUDA(cudaMemcpyAsync(tmp, lvv.data(), lvv.size() * sizeof(double), cudaMemcpyHostToDevice, L->stream));
       if (dense) L->build_dense(tmp);
-      if (integral) L->build_integral(tmp, iplan);
+      if (integral) {
+        const size_t mark = L->owned.size();
+        try {
+          L->build_integral(tmp, iplan);
+        } catch (const Error& e) {
+          // the room was gone when it came to it: the Cholesky form, unless the caller wants this one
+          if (e.code != TCI_ERR_MEMORY || want_form == 3) throw;
+          L->release_after(mark);
+          L->X = nullptr;
+          L->lint = {};
+          integral = false;
+          chol_form = true;
+        }
+      }
       if (chol_form) {
         L->LT = L->alloc(lvv.size());
         dim3 grid((unsigned)((nchol + 31) / 32), (unsigned)((L->npv + 31) / 32));

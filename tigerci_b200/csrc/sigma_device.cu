@@ -23,6 +23,7 @@
 #include <cstring>
 #include <future>
 #include <map>
+#include <set>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -887,6 +888,8 @@ constexpr int RB = 256;     // threads per reduction block
 constexpr int RBLK = 592;   // reduction blocks (4 x 148 SMs)
 // default Davidson subspace budget: the reference's DAVIDSON HARD DRIVE SPACE default of 30 GB
 constexpr double kDefaultSubspaceBytes = 30e9;
+// device bytes left free beside the compact operands of a local deck's two-external step
+constexpr int64_t kOperandMargin = 8000000000;
 // Several contexts may live in one process, driven from different host threads
 // (the request server).  A graph capture on one thread and a cudaFree (which
 // synchronises the device) on another are kept apart by this lock.
@@ -1478,6 +1481,27 @@ struct tci_ctx {
     d.tma_ntiles = tiles;
   }
 
+  // At most so many device bytes the compact integral operands of lower_dom take.
+  static i64 dom_operand_bytes(const Plan& P, const tci::LocalSetup& ls) {
+    const i64 n2 = P.n * P.n;
+    std::vector<i64> dk2h((size_t)P.nD, -1);
+    for (size_t h = 0; h < P.dheads.size(); ++h)
+      for (i64 k = 0; k < P.dheads[h].nD; ++k) dk2h[(size_t)(P.dheads[h].dk0 + k)] = (i64)h;
+    std::set<std::tuple<i64, i64, i64, i64>> seen;  // operand, target head, source head
+    i64 bytes = 0;
+    for (const auto& s : P.sigma_steps) {
+      if (s.kind != STEP_GEMM || s.name != "dd two-external") continue;
+      for (const auto& g : s.gp)
+        for (i64 q = g.seg_begin; q < g.seg_end; ++q) {
+          const GemmSeg& x = s.gs[(size_t)q];
+          const i64 ht = dk2h[(size_t)(g.offC / n2)], hs = dk2h[(size_t)(x.offB / n2)];
+          const i64 mt = ls.dh_len[(size_t)ht], ms = ls.dh_len[(size_t)hs];
+          if (mt > 0 && ms > 0 && seen.insert(std::make_tuple((i64)x.a, x.offA, ht, hs)).second) bytes += 8 * mt * (ms + (ms & 1));
+        }
+    }
+    return bytes;
+  }
+
   // The two-external step of a local deck's plan on the heads' domains: the same problems and segments
   // (target pair matrix, integral matrix x source pair matrix, alpha), each restricted to the target's domain
   // rows, the source's domain as k range and the columns common to both, on compact squares of the local
@@ -1595,7 +1619,7 @@ struct tci_ctx {
     double* abuf = nullptr;
     {
       size_t fr = 0, tot = 0;
-      if (abytes > 0 && cudaMemGetInfo(&fr, &tot) == cudaSuccess && (double)abytes + 8e9 < (double)fr &&
+      if (abytes > 0 && cudaMemGetInfo(&fr, &tot) == cudaSuccess && abytes + kOperandMargin < (i64)fr &&
           dev_malloc(&abuf, (size_t)abytes, stream) == cudaSuccess) {
         owned.push_back(abuf);
         bytes_held += (double)abytes;
@@ -3302,9 +3326,18 @@ int ctx_from_plan(CsfSpace&& sp, Plan&& plan, const double* chol, int64_t device
         ctx->owned.push_back(*p);
       }
       if (!ls->heads7.empty()) {
-        const int64_t opts[4] = {precision, (int64_t)16e9, kblock, 1};
+        // the integrals of the FP64 all-external form leave room for what comes after them: the compact operands of the
+        // two-external step with their margin, and the vectors of a solve of one root
+        int64_t room = 0;
+        if (precision == 0) {
+          size_t fr = 0, tot = 0;
+          TCI_CUDA(cudaMemGetInfo(&fr, &tot));
+          room = std::max<int64_t>(1, (int64_t)fr - ctx->dom_operand_bytes(P, *ls) - kOperandMargin -
+                                          tci_davidson_bytes(std::max<i64>(1, ctx->n_loc), 1, 50, 0));
+        }
+        const int64_t opts[6] = {precision, 0, kblock, 1, 0, room};
         const int rc = tci_local_create(P.nint, P.n, chol, P.nchol, (int64_t)(ls->heads7.size() / 7), ls->heads7.data(),
-                                        ls->dom_idx.data(), ctx->n_loc, device, opts, 4, &ctx->loc_allext);
+                                        ls->dom_idx.data(), ctx->n_loc, device, opts, 6, &ctx->loc_allext);
         if (rc != TCI_OK) throw Error(rc, "pair-domain all-external set-up failed");
       }
       TCI_CUDA(cudaSetDevice(ctx->device));

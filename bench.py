@@ -520,6 +520,26 @@ def molecular_cpu(mol):
             "what": "oracle Davidson (davidson.f90 restated) over the integral-direct CPU sigma"}
 
 
+def local_work(precision, st, t, bf16):
+    """The work and rate of one pair-domain application of t seconds: those of the form that ran (LocalAllExternal.stats)."""
+    fl, kern = {
+        "dense": (st["dense_flops"],
+                  "allext_tf32x3_kernel (dense padded W+/W- over all external pairs, tcgen05 kind::tf32, 3xTF32)"),
+        "integral": (st["integral_flops"], "local_integral (packed integrals on the domains, mma.sync m8n8k4 f64)"),
+        "cholesky": (st["flops"], "tma_gemm (grouped 3xTF32, pair-domain Cholesky form)" if precision == "tf32x3" else
+                     "gemm_mma_f64 (pair-domain Cholesky form, mma.sync m8n8k4 f64)"),
+    }[st["form"]]
+    # 3xTF32 issues three MMAs per product: its FP32-accurate peak is a third of the TF32 peak (half the measured dense
+    # BF16 figure)
+    peak = bf16 / 2 / 3 if precision == "tf32x3" else None
+    # the dense form pads each block to all externals, the integral form the columns and rows of a domain: only the
+    # Cholesky form's flops are all useful
+    return {"useful_tflops": fl / t / 1e12 if st["form"] == "cholesky" else None, "flops_per_apply": fl,
+            "roofline": {"kernel": kern, "bound": "tensor", "achieved": fl / t / 1e12, "peak": peak, "unit": "TFLOP/s",
+                         "frac": (fl / t / 1e12 / peak) if peak else None,
+                         "peak_kind": "3xTF32: measured dense BF16 / 2 / 3" if peak else None}}
+
+
 def local_measure(n_pairs, device, hbm, bf16, steps=3, warmup=3, nchol=2400, forms=("tf32x3", "fp64"), n_virt=400):
     """All-external term over uneven pair domains: n_pairs internal pairs (35
     doubly occupied internal orbitals), domains of 20..180 of 400 external
@@ -558,25 +578,11 @@ def local_measure(n_pairs, device, hbm, bf16, steps=3, warmup=3, nchol=2400, for
         torch.cuda.synchronize()
         t = sum(a.elapsed_time(b) for a, b in ev) / 1e3 / n_steps
         sig[form] = s.cpu().numpy()
-        # 3xTF32 issues three MMAs per product: its FP32-accurate peak is a third of the TF32 peak
-        # (half the measured dense BF16 figure)
-        peak = bf16 / 2 / 3 if form == "tf32x3" else None
-        # the form applied: the Cholesky form's flops are the useful work; the dense form does its own
-        # (padded) flops on the all-external kernel, and those set its tensor roofline
-        fl = st["dense_flops"] if st["form"] == "dense" else st["flops"]
-        kern = ("allext_tf32x3_kernel (dense padded W+/W- over all external pairs, tcgen05 kind::tf32, 3xTF32)"
-                if st["form"] == "dense" else
-                "tma_gemm (grouped 3xTF32, pair-domain Cholesky form)" if form == "tf32x3" else
-                "gemm_f64 grouped (pair-domain Cholesky form, FP64)")
-        out[form] = {"ms_per_apply": 1e3 * t, "form": st["form"], "useful_tflops": st["flops"] / t / 1e12,
-                     "flops_per_apply": fl, "cholesky_form_flops": st["flops"],
-                     "cholesky_form_setup_ms": st["tuned_ms"], "dense_form_setup_ms": st["dense_ms"] or None,
+        out[form] = {"ms_per_apply": 1e3 * t, "form": st["form"], "cholesky_form_flops": st["flops"],
+                     "cholesky_form_setup_ms": st["tuned_ms"] or None, "dense_form_setup_ms": st["dense_ms"] or None,
                      "chunk": int(st["chunk"]), "tile_cfg": int(st["tile_cfg"]),
                      "autotune_candidates": int(st["candidates"]), "device_gb": st["device_bytes"] / 1e9,
-                     "init_s": init_s,
-                     "roofline": {"kernel": kern, "bound": "tensor", "achieved": fl / t / 1e12, "peak": peak,
-                                  "unit": "TFLOP/s", "frac": (fl / t / 1e12 / peak) if peak else None,
-                                  "peak_kind": "3xTF32: measured dense BF16 / 2 / 3" if peak else None}}
+                     "init_s": init_s, **local_work(form, st, t, bf16)}
         if st["form"] == "dense":
             # the W tiles are streamed once per group of 64 CI blocks of each operator
             out[form]["w_gb"] = st["dense_w_bytes"] / 1e9

@@ -370,13 +370,15 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
 int tci_local_apply(tci_local* loc, const double* d_c, double* d_sigma, int64_t n, void* stream);
 /* The same with host arrays. */
 int tci_local_apply_host(tci_local* loc, const double* c, double* sigma, int64_t n);
-/* out[len], len >= 9, up to 13: flops per application (4 nchol sum n^3 over
- * head spin functions), gathered Cholesky bytes per application, device
- * bytes, chunk size, FP64 tile shape of the second GEMM, autotuned time (ms),
- * autotuner candidates, last host application (ms), head spin-function
- * blocks, form applied (0 Cholesky, 1 dense, 2 integrals), the dense form's set-up time
+/* out[len], len >= 9, up to 15: the Cholesky form's flops per application
+ * (4 nchol sum n^3 over head spin functions) and gathered Cholesky bytes,
+ * device bytes, chunk size, tile width of the Cholesky form's first GEMM in
+ * the mixed precision (0: 128, 1: 64), autotuned time (ms), autotuner
+ * candidates, last host application (ms), head spin-function blocks, form
+ * applied (0 Cholesky, 1 dense, 2 integrals), the dense form's set-up time
  * (ms, 0 if not timed), its flops (2 np^2 per singlet-coupled and 2 nm^2 per
- * triplet-coupled block), its W tile bytes. */
+ * triplet-coupled block), its W tile bytes, the integral form's flops (its
+ * products, padded columns included) and copies of sigma (0 in other forms). */
 int tci_local_stats(const tci_local* loc, double* out, int64_t len);
 void tci_local_destroy(tci_local* loc);
 

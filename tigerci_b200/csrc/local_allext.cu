@@ -316,6 +316,7 @@ struct tci_local {
   int form = 0;              // form in use: 0 Cholesky, 1 dense, 2 integrals on the domains (FP64)
   double* X = nullptr;       // form 2: (ab|cd), npv x npv
   tci_lint::Device lint;
+  double integral_flops = 0;  // form 2: products of one application, padding included, times two
   bool dense_ready = false;  // the dense operators are built
   int64_t np_d = 0, nm_d = 0, nsing_d = 0, ntrip_d = 0;
   float *w32p = nullptr, *w32m = nullptr, *u2p = nullptr, *u2m = nullptr;
@@ -952,7 +953,10 @@ int tci_local_create(int64_t num_internal, int64_t num_external, const double* c
       L->tuned_ms = best;
       if (pick != std::make_pair(L->jc, L->cfg2)) L->configure(pick.first, pick.second);
     }
-    if (integral) L->configure_form(2);
+    if (integral) {
+      L->integral_flops = iplan.flops;
+      L->configure_form(2);
+    }
     if (L->dense_ready) {
       L->configure_form(1);
       L->time_once();
@@ -1016,10 +1020,11 @@ int tci_local_apply_host(tci_local* L, const double* c, double* sigma, int64_t n
 
 int tci_local_stats(const tci_local* L, double* out, int64_t len) {
   if (!L || !out || len < 9) return TCI_ERR_ARG;
-  const double v[13] = {L->flops,       L->lbytes,           L->dev_bytes,   (double)L->jc,    (double)L->cfg2,
+  const double v[15] = {L->flops,       L->lbytes,           L->dev_bytes,   (double)L->jc,    (double)L->cfg2,
                         L->tuned_ms,    (double)L->candidates, L->last_ms,   (double)L->blocks.size(),
-                        (double)L->form, L->dense_ms,        L->dense_flops, L->dense_bytes};
-  std::memcpy(out, v, sizeof(double) * (size_t)std::min<int64_t>(len, 13));
+                        (double)L->form, L->dense_ms,        L->dense_flops, L->dense_bytes,
+                        L->integral_flops, L->form == 2 ? (double)L->lint.parts : 0.0};
+  std::memcpy(out, v, sizeof(double) * (size_t)std::min<int64_t>(len, 15));
   return TCI_OK;
 }
 

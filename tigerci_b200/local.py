@@ -71,11 +71,12 @@ class LocalAllExternal:
     def stats(self) -> dict:
         """form: "cholesky", "dense" or "integral" (the one applied); tuned_ms / dense_ms: the set-up timings of the two forms
         (0 where a form was not timed); flops: the Cholesky form's 4 nchol sum n^3, dense_flops: the dense form's
-        2 np^2 per singlet-coupled and 2 nm^2 per triplet-coupled block; dense_w_bytes: its FP32 W tiles."""
-        out = np.zeros(13)
-        check(self._L.tci_local_stats(self._h, ptr(out), 13))
+        2 np^2 per singlet-coupled and 2 nm^2 per triplet-coupled block; dense_w_bytes: its FP32 W tiles; integral_flops,
+        integral_parts: the integral form's products (padded columns included) times two and its copies of sigma."""
+        out = np.zeros(15)
+        check(self._L.tci_local_stats(self._h, ptr(out), 15))
         keys = ["flops", "cholesky_bytes", "device_bytes", "chunk", "tile_cfg", "tuned_ms", "candidates", "last_ms",
-                "blocks", "form", "dense_ms", "dense_flops", "dense_w_bytes"]
+                "blocks", "form", "dense_ms", "dense_flops", "dense_w_bytes", "integral_flops", "integral_parts"]
         d = dict(zip(keys, out.tolist()))
         d["form"] = ("cholesky", "dense", "integral")[int(d["form"])]
         return d

@@ -20,7 +20,9 @@
 // eight warps share 64-deep slices of tiles down to 16 x 16. 32 problems of 35 x 35 x (40 x 35): 76 us with four
 // warps, 32-deep slices and 64-row tiles, 48 us so; 64 of 53 x 53 x (40 x 53): 98 -> 83 us.
 #include <algorithm>
+#include <array>
 #include <cmath>
+#include <map>
 #include <mutex>
 #include <stdexcept>
 #include <type_traits>
@@ -454,9 +456,25 @@ namespace tci_dmma {
 Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& segs) {
   // the longest problems first: the short ones fill the last wave
   std::vector<Form> forms;
-  std::vector<size_t> order;
+  std::vector<size_t> order, kind;
+  // problems of one shape and form are placed alike: looked at once, with the longest k (a plan has hundreds of them)
+  struct Kind {
+    DGemmProblem g;
+    Form f;
+    double count;
+  };
+  std::vector<Kind> kinds;
+  std::map<std::array<long long, 3>, size_t> seen;
   for (size_t i = 0; i < pr.size(); ++i) {
-    forms.push_back(form(pr[i], segs));
+    const Form f = form(pr[i], segs);
+    const long long flags = f.a_k | f.a_r << 1 | f.b_k << 2 | f.b_r << 3 | f.a_even << 4 | f.b_even << 5;
+    const auto at = seen.insert({{pr[i].M, pr[i].N, flags}, kinds.size()});
+    if (at.second) kinds.push_back(Kind{pr[i], f, 0});
+    Kind& x = kinds[at.first->second];
+    x.count += 1;
+    x.f.k = std::max(x.f.k, f.k);
+    kind.push_back(at.first->second);
+    forms.push_back(f);
     order.push_back(i);
   }
   std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return forms[a].k > forms[b].k; });
@@ -473,9 +491,9 @@ Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& seg
   double best_time = 0;
   for (const Try& y : {best, Try{8, 12, 1.12}, Try{8, 8, 1.25}, Try{8, NB, 1.6}, Try{4, NB, 1.6}, Try{3, 3, 1.6}, Try{2, 2, 1.6}}) {
     double work = 0, n = 0;
-    for (size_t i = 0; i < pr.size(); ++i) {
-      const Place x = place(pr[i], forms[i], y.bmb, y.bnb);
-      n += (double)(x.c.tm * x.c.tn);
+    for (const Kind& q : kinds) {
+      const Place x = place(q.g, q.f, y.bmb, y.bnb);
+      n += q.count * (double)(x.c.tm * x.c.tn);
       work = std::max(work, x.work);
     }
     const double time = std::ceil(n / sms) * work * y.slow;
@@ -485,9 +503,11 @@ Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& seg
     }
     if (n > 16 * sms) break;
   }
+  std::vector<Place> places;
+  for (const Kind& q : kinds) places.push_back(place(q.g, q.f, best.bmb, best.bnb));
   Tiles t;
   for (size_t i : order) {
-    const Place x = place(pr[i], forms[i], best.bmb, best.bnb);
+    const Place& x = places[kind[i]];
     DGemmProblem g = pr[i];
     g.trans_c = (x.swapped ? 1 : 0) | 2 * x.c.tm;
     g.tiles_n = x.c.tn;

@@ -28,6 +28,21 @@ struct Tables {
     return k;
   }
 };
+// The device copies of a launch's problems, all classes in one table; up: uploads a vector of problems.
+template <class Upload>
+Tables tables(const Tiles& t, Upload&& up) {
+  std::vector<tci_dev::DGemmProblem> all;
+  for (const auto& p : t.probs) all.insert(all.end(), p.begin(), p.end());
+  tci_dev::DGemmProblem* d = up(all);
+  Tables x;
+  for (int c = 0; c < CLASSES; ++c) {
+    x.probs[c] = d;
+    x.nprob[c] = (int)t.probs[c].size();
+    x.ntiles[c] = t.ntiles[c];
+    d += t.probs[c].size();
+  }
+  return x;
+}
 // All classes of a launch, segs the table its problems index.
 cudaError_t launch(const Tables& t, const tci_dev::DGemmSeg* segs, cudaStream_t st);
 

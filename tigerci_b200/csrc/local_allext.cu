@@ -401,12 +401,7 @@ struct tci_local {
       std::vector<DGemmProblem> pr;
       std::vector<DGemmSeg> sg;
       tci_dev::tile_problems(v, 64, 64, false, pr, sg);
-      const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
-      for (int c = 0; c < tci_dmma::CLASSES; ++c) {
-        g.t.probs[c] = upload(t.probs[c]);
-        g.t.nprob[c] = (int)t.probs[c].size();
-        g.t.ntiles[c] = t.ntiles[c];
-      }
+      g.t = tci_dmma::tables(tci_dmma::tile(pr, sg), [&](const auto& x) { return upload(x); });
       g.segs = upload(sg);
     };
     finish(v1, a);
@@ -545,12 +540,7 @@ struct tci_local {
       sg.push_back(DGemmSeg{lpk + r * nchol, lpk, nchol, nchol, nchol, 0, 1, 1.0});
     }
     GemmLaunch g;
-    const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
-    for (int c = 0; c < tci_dmma::CLASSES; ++c) {
-      g.t.probs[c] = upload(t.probs[c]);
-      g.t.nprob[c] = (int)t.probs[c].size();
-      g.t.ntiles[c] = t.ntiles[c];
-    }
+    g.t = tci_dmma::tables(tci_dmma::tile(pr, sg), [&](const auto& x) { return upload(x); });
     g.segs = upload(sg);
     launch_gemm(g);
     LCUDA(tci_lint::mirror(X, npv, stream));

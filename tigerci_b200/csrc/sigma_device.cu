@@ -2052,14 +2052,7 @@ struct tci_ctx {
   }
 
   tci_dmma::Tables mma_tables(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& sg) {
-    const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
-    tci_dmma::Tables d;
-    for (int c = 0; c < tci_dmma::CLASSES; ++c) {
-      d.probs[c] = upload(t.probs[c], owned, stream);
-      d.nprob[c] = (int)t.probs[c].size();
-      d.ntiles[c] = t.ntiles[c];
-    }
-    return d;
+    return tci_dmma::tables(tci_dmma::tile(pr, sg), [&](const auto& v) { return upload(v, owned, stream); });
   }
 
   DevStep lower(const Step& s) {

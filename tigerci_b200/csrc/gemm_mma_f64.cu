@@ -1,7 +1,9 @@
 // FP64 grouped GEMM on the double-precision matrix instruction (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind):
 // C (M x N) = beta C + sum over a problem's segments of alpha op(A) op(B), any leading dimension and 8-byte
 // alignment, the problem / segment tables of gemm_tables.h. The instruction is a chain of four fmas in ascending k, so
-// every sum is the one a scalar kernel makes: segments in table order, k ascending, alpha on op(B).
+// where the warps share a tile's columns every sum is the one a scalar kernel makes: segments in table order, k ascending,
+// alpha on op(B) (on op(A) where the operands change places); where eight warps share k each sums every eighth group of 8 k
+// and the eight sums are added in warp order.
 //
 // Bound by the FP64 pipe: the instruction runs at 37 TFLOP/s on this part, the same as scalar fma, but one operand
 // word read from shared memory feeds eight products instead of four or eight registers' worth of broadcasts, so the

@@ -8,8 +8,9 @@
 
 namespace tci_dmma {
 
-// Problems sorted into the kernel's tile classes: the shape of a tile and how its four warps share it (rows and
-// columns, or k slices where a launch has too few tiles) x the two storage orders of the column operand.
+// Problems sorted into the kernel's tile classes: six pairs of operand modes (storage order and copy width of the row and
+// the column operand) x two work splits (four warps share a tile's columns, or eight share k where a launch has too few
+// tiles) x one to eight 8-row blocks of a tile.
 constexpr int CLASSES = 96;
 struct Tiles {
   std::vector<tci_dev::DGemmProblem> probs[CLASSES];

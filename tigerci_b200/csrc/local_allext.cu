@@ -28,8 +28,9 @@
 // (unpack, chunks, pack) is captured as one CUDA graph.
 //
 // In FP64 the packed integrals X = Lpk Lpk^T over all externals replace the
-// Cholesky vectors where they pay (local_integral.cu): n_h^4 / 2 products per
-// block on the domain instead of 4 nchol n_h^3, bound by one streaming of X.
+// Cholesky vectors where they pay (local_integral.cu): n^2 n_h^2 flops per block
+// (n externals in all: the blocks are padded with zeros) instead of
+// 4 nchol n_h^3, bound by the copies of the packed rows and the products together.
 //
 // In the mixed form a second, dense form competes with it: the packed
 // integral form of the non-local all-external term (W+ over the pairs (aa)

@@ -60,8 +60,8 @@ TOL_RESIDUAL, TOL_ENERGY = 1e-6, 1e-8
 # every run of this benchmark's own arm (solves.fp64.iterations); the reference arm has no GPU to count them
 SIGMA_BUILDS_PER_SOLVE = 27
 # ncu DRAM bytes (read + write) of one launch over its algorithmic bytes (the W operators): FP64 split-K
-# all-external at 120 virtuals 863.3 MB / 829.5 MB; tcgen05 all-external at 140 virtuals 809.9 MB / 773.4 MB
-TRAFFIC_RATIO = {"fp64": 863.26 / 829.498, "tf32x3": (800.509 + 9.346) / 773.381}
+# all-external at 120 virtuals 871.1 MB / 829.5 MB; tcgen05 all-external at 140 virtuals 811.7 MB / 773.4 MB
+TRAFFIC_RATIO = {"fp64": (409.748 + 424.122 + 16.697 + 20.508) / 829.498, "tf32x3": (800.377 + 11.360) / 773.381}
 TRAFFIC_SOURCE = {"fp64": "ncu dram read+write ratio at 120 virtuals x full-size bytes",
                   "tf32x3": "ncu dram read+write ratio at 140 virtuals x full-size bytes"}
 

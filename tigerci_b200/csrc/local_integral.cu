@@ -14,7 +14,7 @@
 // stages, or two of 32 k, are no faster: 13.7, 14.4).  The zero
 // padding inside a column costs 1 / density in d and b, but nothing is gathered: the index arithmetic of a
 // gathering kernel (lanes over the domain, integrals from shared memory) cost more than the padding (30 ms against
-// 15.4 for the form with eight warps doing both), and n^2 sum n_h^2 products replace the Cholesky form's 4 nchol sum n_h^3.
+// 15.4 for the form with eight warps doing both), and n^2 sum n_h^2 flops replace the Cholesky form's 4 nchol sum n_h^3.
 // Bound by the copies (9.9 ms alone) and the products of half-filled tiles (11.4 alone) together.  Every sum in a fixed order.
 #include <algorithm>
 #include <limits>

@@ -272,6 +272,13 @@ int tci_selftest_gemm_f64(int64_t device, int64_t M, int64_t N, int64_t K, int64
                           int64_t lda, int64_t ldb, int64_t ldc, int64_t a_off, int64_t b_off, int64_t a_step,
                           int64_t b_step, double alpha, double beta, const double* A, int64_t na, const double* B,
                           int64_t nb, double* C);
+/* nprob products C_p = op(A_p) op(B_p) of one launch of it, the matrices one
+ * after the other, each from an even element on, rows pad longer than their
+ * data (C: none).  tiles[102] = the tiles of each tile class; device < 0: only
+ * these, on the host alone. */
+int tci_selftest_gemm_f64_group(int64_t device, int64_t nprob, const int64_t* M, const int64_t* N, const int64_t* K,
+                                int64_t tA, int64_t tB, int64_t pad, const double* A, int64_t na, const double* B,
+                                int64_t nb, double* C, int64_t nc, int64_t* tiles);
 /* Its address arithmetic, on the host alone: the asynchronous copies that a
  * block of tile class cls (0 .. 95: operand modes x work split x row blocks)
  * makes of one segment's row (which 0) or column (1) operand, nr rows of the

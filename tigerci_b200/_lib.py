@@ -65,6 +65,7 @@ EXPORTS = [
     "tci_selftest_mma_rate",
     "tci_selftest_gemm_f64",
     "tci_selftest_gemm_f64_copies",
+    "tci_selftest_gemm_f64_group",
     "tci_selftest_com",
     "tci_selftest_integral_plan",
     "tci_selftest_local_alloc_limit",
@@ -178,6 +179,7 @@ def lib():
         L.tci_selftest_gemm_f64_copies.argtypes = [i64] * 7 + [P]
         L.tci_selftest_integral_plan.argtypes = [i64, i64, P, P, P, i64, i64, P]
         L.tci_selftest_local_alloc_limit.argtypes = [i64]
+        L.tci_selftest_gemm_f64_group.argtypes = [i64, i64, P, P, P, i64, i64, i64, P, i64, P, i64, P, i64, P]
         L.tci_selftest_com.argtypes = [i64, i64, i64, P, i64, P, P, P, P, P, i64, P]
         L.tci_operator_from_records.argtypes = [i64, i64, P, P, i64, P]
         L.tci_reference_weight.argtypes = [P, P, i64, P]

@@ -178,7 +178,8 @@ struct Shape {
   static constexpr size_t smem = sizeof(double) * (size_t)STAGE * STG;
 };
 
-template <int MB, int WK, Mode AM, Mode BM_>
+// ANY: tiles of 1 to MB row blocks in one launch, else of MB or MB - 1.
+template <int MB, int WK, Mode AM, Mode BM_, bool ANY>
 __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS)) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
                                                       const DGemmSeg* __restrict__ segs) {
   using Sh = Shape<MB, WK, AM, BM_>;
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
   const int mblk = (int)((rows + 7) >> 3), nblk = (int)((cols + 7) >> 3), tm = (int)(P.trans_c >> 1);
   const int mq = mblk / tm, mr = mblk % tm, nq = nblk / tn, nr = nblk % tn;
   const long long m0 = 8ll * (ti * mq + min(ti, mr)), n0 = 8ll * (tj * nq + min(tj, nr));
-  const int mb = mq + (ti < mr ? 1 : 0), nbt = nq + (tj < nr ? 1 : 0);  // mb: MB or MB - 1
+  const int mb = mq + (ti < mr ? 1 : 0), nbt = nq + (tj < nr ? 1 : 0);  // mb: MB or MB - 1, ANY: 1 .. MB
   const int mrows = (int)min((long long)(8 * mb), rows - m0), ncols = (int)min((long long)(8 * nbt), cols - n0);
   // this warp's column blocks of the tile
   const int j0 = WK == 1 ? (nbt * role) >> 2 : 0, nb = WK == 1 ? ((nbt * (role + 1)) >> 2) - j0 : nbt;
@@ -319,8 +320,20 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
       else if (nb == 2) body(rr, std::integral_constant<int, 2>());
       else if (nb == 1) body(rr, std::integral_constant<int, 1>());
     };
-    if (mb == MB) bodies(std::integral_constant<int, MB>());
-    else bodies(std::integral_constant<int, MB - 1>());
+    if (mb == MB) {
+      bodies(std::integral_constant<int, MB>());
+    } else if constexpr (ANY) {
+      static_assert(MB == 8, "every height has its body");
+      if (mb == 7) bodies(std::integral_constant<int, 7>());
+      else if (mb == 6) bodies(std::integral_constant<int, 6>());
+      else if (mb == 5) bodies(std::integral_constant<int, 5>());
+      else if (mb == 4) bodies(std::integral_constant<int, 4>());
+      else if (mb == 3) bodies(std::integral_constant<int, 3>());
+      else if (mb == 2) bodies(std::integral_constant<int, 2>());
+      else bodies(std::integral_constant<int, 1>());
+    } else {
+      bodies(std::integral_constant<int, MB - 1>());
+    }
     st = st == STG - 1 ? 0 : st + 1;
   }
   cp_wait<0>();
@@ -363,7 +376,7 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
   }
 }
 
-template <int MB, int WK, Mode AM, Mode BM_>
+template <int MB, int WK, Mode AM, Mode BM_, bool ANY = false>
 cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles, cudaStream_t st) {
   constexpr size_t smem = Shape<MB, WK, AM, BM_>::smem;
   static_assert(WK == 1 || smem >= sizeof(double2) * WK * MB * NB * 32, "the warps' sums fit the stages");
@@ -373,20 +386,26 @@ cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long 
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::call_once(once[dev], [&] {
-    cudaFuncSetAttribute(gemm_mma_f64<MB, WK, AM, BM_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gemm_mma_f64<MB, WK, AM, BM_, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
-  gemm_mma_f64<MB, WK, AM, BM_><<<(unsigned)ntiles, threads(WK), smem, st>>>(probs, nprob, segs);
+  gemm_mma_f64<MB, WK, AM, BM_, ANY><<<(unsigned)ntiles, threads(WK), smem, st>>>(probs, nprob, segs);
   return cudaGetLastError();
 }
 
 using Go = cudaError_t (*)(const DGemmProblem*, int, const DGemmSeg*, long long, cudaStream_t);
-// one F per class
+// one F per row class
 #define TCI_ROWS(F, WK, A, B) \
   F<1, WK, A, B>, F<2, WK, A, B>, F<3, WK, A, B>, F<4, WK, A, B>, F<5, WK, A, B>, F<6, WK, A, B>, F<7, WK, A, B>, F<8, WK, A, B>
 #define TCI_PAIR(F, A, B) TCI_ROWS(F, 1, A, B), TCI_ROWS(F, 8, A, B)
 #define TCI_CLASSES(F) \
   TCI_PAIR(F, K16, K16), TCI_PAIR(F, K16, R16), TCI_PAIR(F, K8, K8), TCI_PAIR(F, K8, R16), TCI_PAIR(F, RT8, K8), TCI_PAIR(F, RT8, R16)
-constexpr Go kGo[tci_dmma::CLASSES] = {TCI_CLASSES(go)};
+constexpr Go kGo[tci_dmma::CLASSES] = {TCI_CLASSES(go),
+                                       go<8, 1, K16, K16, true>,
+                                       go<8, 1, K16, R16, true>,
+                                       go<8, 1, K8, K8, true>,
+                                       go<8, 1, K8, R16, true>,
+                                       go<8, 1, RT8, K8, true>,
+                                       go<8, 1, RT8, R16, true>};
 
 // Tile counts of a problem of rows x cols: at most bmb row blocks x bnb column blocks.
 struct Cut {
@@ -507,6 +526,26 @@ Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& seg
   }
   std::vector<Place> places;
   for (const Kind& q : kinds) places.push_back(place(q.g, q.f, best.bmb, best.bnb));
+  // The heights of a mode pair run one after another, a launch each. Where those launches are short (problems of many sizes,
+  // few tiles of each, a long k: the second product of 30 pair domains of 60-150 externals, 18 + 28 + 74 + 27 tiles, 16.5 ms
+  // in four launches, 5.6 in one; the scalar kernel's one launch 10) one launch for all of them: its time by the same rule,
+  // with a margin for the two blocks per SM and registers of the highest tile that all its tiles have.
+  for (int m = 0; m < 6; ++m) {
+    double n[8] = {}, work[8] = {}, all = 0, longest = 0, apart = 0;
+    for (size_t i = 0; i < kinds.size(); ++i) {
+      const Place& x = places[i];
+      if (x.cls / 8 != 2 * m) continue;  // eight warps sharing k, or another pair
+      const double tiles = kinds[i].count * (double)(x.c.tm * x.c.tn);
+      n[x.cls % 8] += tiles;
+      work[x.cls % 8] = std::max(work[x.cls % 8], x.work);
+      all += tiles;
+      longest = std::max(longest, x.work);
+    }
+    for (int c = 0; c < 8; ++c) apart += std::ceil(n[c] / sms) * work[c];
+    if (std::ceil(all / sms) * longest < 0.8 * apart)
+      for (Place& x : places)
+        if (x.cls < ROW_CLASSES && x.cls / 8 == 2 * m) x.cls = ROW_CLASSES + m;
+  }
   Tiles t;
   for (size_t i : order) {
     const Place& x = places[kind[i]];
@@ -566,11 +605,11 @@ void copies_of(int which, int nr, long long K, long long ld, long long off, long
   else all(typename Sh::B());
 }
 using CopiesOf = void (*)(int, int, long long, long long, long long, long long, int64_t*);
-constexpr CopiesOf kCopies[tci_dmma::CLASSES] = {TCI_CLASSES(copies_of)};
+constexpr CopiesOf kCopies[tci_dmma::ROW_CLASSES] = {TCI_CLASSES(copies_of)};
 }  // namespace
 extern "C" int tci_selftest_gemm_f64_copies(int64_t cls, int64_t which, int64_t nr, int64_t K, int64_t ld, int64_t off,
                                             int64_t len, int64_t* out) {
-  if (!out || cls < 0 || cls >= tci_dmma::CLASSES || which < 0 || which > 1 || nr < 1 || K < 1 || ld < 1 || off < 0)
+  if (!out || cls < 0 || cls >= tci_dmma::ROW_CLASSES || which < 0 || which > 1 || nr < 1 || K < 1 || ld < 1 || off < 0)
     return TCI_ERR_ARG;
   out[0] = out[1] = out[2] = 0;
   kCopies[cls]((int)which, (int)nr, K, ld, off, len, out);
@@ -620,6 +659,72 @@ extern "C" int tci_selftest_gemm_f64(int64_t device, int64_t M, int64_t N, int64
       if (rc == TCI_OK) ok(tci_dmma::launch(d, ds, 0));
       ok(cudaDeviceSynchronize());
       ok(cudaMemcpy(C, dC, cb, cudaMemcpyDeviceToHost));
+    }
+  } catch (...) {
+    rc = TCI_ERR_INTERNAL;
+  }
+  for (void* p : {(void*)dA, (void*)dB, (void*)dC, (void*)ds, (void*)dp}) cudaFree(p);
+  return rc;
+}
+
+// Test entry: nprob products C_p (M x N) = op(A_p) op(B_p) of one launch, the matrices one after the other from 16-byte
+// aligned places, leading dimensions pad above the rows' lengths. tiles[CLASSES]: the tiles of each class; device < 0: only
+// these.
+extern "C" int tci_selftest_gemm_f64_group(int64_t device, int64_t nprob, const int64_t* M, const int64_t* N, const int64_t* K,
+                                           int64_t tA, int64_t tB, int64_t pad, const double* A, int64_t na, const double* B,
+                                           int64_t nb, double* C, int64_t nc, int64_t* tiles) {
+  if (nprob < 1 || !M || !N || !K || pad < 0 || !tiles || (device >= 0 && (!A || !B || !C))) return TCI_ERR_ARG;
+  double *dA = nullptr, *dB = nullptr, *dC = nullptr;
+  DGemmSeg* ds = nullptr;
+  DGemmProblem* dp = nullptr;
+  int rc = TCI_OK;
+  auto ok = [&](cudaError_t e) {
+    if (e != cudaSuccess && rc == TCI_OK) rc = TCI_ERR_CUDA;
+    return rc == TCI_OK;
+  };
+  try {
+    int64_t ea = 0, eb = 0, ec = 0;
+    auto take = [](int64_t& at, int64_t rows, int64_t ld) {
+      const int64_t o = at;
+      at += (rows * ld + 1) / 2 * 2;
+      return o;
+    };
+    std::vector<int64_t> oa, ob, oc;
+    for (int64_t p = 0; p < nprob; ++p) {
+      if (M[p] < 1 || N[p] < 1 || K[p] < 1) return TCI_ERR_ARG;
+      oa.push_back(take(ea, tA ? K[p] : M[p], (tA ? M[p] : K[p]) + pad));
+      ob.push_back(take(eb, tB ? N[p] : K[p], (tB ? K[p] : N[p]) + pad));
+      oc.push_back(take(ec, M[p], N[p]));
+    }
+    if (device >= 0) {
+      if (ea > na || eb > nb || ec > nc) return TCI_ERR_ARG;
+      if (ok(cudaSetDevice((int)device)) && ok(cudaMalloc(&dA, sizeof(double) * (size_t)ea)) &&
+          ok(cudaMalloc(&dB, sizeof(double) * (size_t)eb)) && ok(cudaMalloc(&dC, sizeof(double) * (size_t)ec)) &&
+          ok(cudaMalloc(&ds, sizeof(DGemmSeg) * (size_t)nprob)))
+        ok(cudaMalloc(&dp, sizeof(DGemmProblem) * (size_t)nprob));
+    }
+    if (rc == TCI_OK) {
+      std::vector<DGemmProblem> pr;
+      std::vector<DGemmSeg> sg;
+      for (int64_t p = 0; p < nprob; ++p) {
+        pr.push_back(DGemmProblem{dC + oc[p], N[p], M[p], N[p], 0, 0, 0.0, p, p + 1, 0});
+        sg.push_back(DGemmSeg{dA + oa[p], dB + ob[p], (tA ? M[p] : K[p]) + pad, (tB ? K[p] : N[p]) + pad, K[p], tA ? 1 : 0,
+                              tB ? 1 : 0, 1.0});
+      }
+      const tci_dmma::Tiles t = tci_dmma::tile(pr, sg);
+      for (int c = 0; c < tci_dmma::CLASSES; ++c) tiles[c] = t.ntiles[c];
+      if (device >= 0) {
+        const tci_dmma::Tables d = tci_dmma::tables(t, [&](const std::vector<DGemmProblem>& v) {
+          ok(cudaMemcpy(dp, v.data(), sizeof(DGemmProblem) * v.size(), cudaMemcpyHostToDevice));
+          return dp;
+        });
+        ok(cudaMemcpy(ds, sg.data(), sizeof(DGemmSeg) * sg.size(), cudaMemcpyHostToDevice));
+        ok(cudaMemcpy(dA, A, sizeof(double) * (size_t)ea, cudaMemcpyHostToDevice));
+        ok(cudaMemcpy(dB, B, sizeof(double) * (size_t)eb, cudaMemcpyHostToDevice));
+        if (rc == TCI_OK) ok(tci_dmma::launch(d, ds, 0));
+        ok(cudaDeviceSynchronize());
+        if (rc == TCI_OK) ok(cudaMemcpy(C, dC, sizeof(double) * (size_t)ec, cudaMemcpyDeviceToHost));
+      }
     }
   } catch (...) {
     rc = TCI_ERR_INTERNAL;

@@ -60,3 +60,23 @@ def test_against_numpy(tA, tB, pad, need_gpu):
         c = got[oc[p]:][: m * n].reshape(m, n)
         # K products and sums on either side, of at most |a||b|
         assert (np.abs(c - a @ b) <= 2 * (k + 4) * 2.0 ** -53 * (np.abs(a) @ np.abs(b))).all(), (p, m, n, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tA", [0, 1])
+@pytest.mark.parametrize("tB", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(35, 35, 35), (53, 57, 130), (64, 128, 200), (33, 129, 500), (128, 40, 67), (40, 24, 1000), (30, 48, 63)])
+def test_sums_do_not_depend_on_the_launch(tA, tB, M, N, K, need_gpu):
+    """One product alone, on few tiles, and six hundred copies of it, which fill the chip: the same sums bit for bit."""
+    rng = np.random.default_rng(M + N)
+    one, many = [], 600
+    for rows, cols in ((K, M) if tA else (M, K), (N, K) if tB else (K, N)):
+        x = np.zeros((rows * cols + 1) // 2 * 2)
+        x[: rows * cols] = rng.uniform(-0.5, 0.5, rows * cols)
+        one.append(x)
+    ec = (M * N + 1) // 2 * 2
+    alone, filled = np.zeros(ec), np.zeros(many * ec)
+    ta = _run(0, [M], [N], [K], tA, tB, 0, one[0], one[1], alone)
+    tm = _run(0, many * [M], many * [N], many * [K], tA, tB, 0, np.tile(one[0], many), np.tile(one[1], many), filled)
+    assert (np.flatnonzero(ta)[0] % 16 >= 8) and (np.flatnonzero(tm)[0] % 16 < 8)  # both work splits
+    assert (filled.reshape(many, ec) == alone).all()

@@ -1,9 +1,9 @@
 // FP64 grouped GEMM on the double-precision matrix instruction (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind):
 // C (M x N) = beta C + sum over a problem's segments of alpha op(A) op(B), any leading dimension and 8-byte
-// alignment, the problem / segment tables of gemm_tables.h. The instruction is a chain of four fmas in ascending k, so
-// where the warps share a tile's columns every sum is the one a scalar kernel makes: segments in table order, k ascending,
-// alpha on op(B) (on op(A) where the operands change places); where eight warps share k each sums every eighth group of 8 k
-// and the eight sums are added in warp order.
+// alignment, the problem / segment tables of gemm_tables.h. The instruction is a chain of four fmas in ascending k and every
+// element is one chain, so every sum is the one a scalar kernel makes, whatever tile and work split a launch takes: segments
+// in table order, k ascending, alpha on op(B) (on op(A) where the operands change places). Mixed-precision solves need that:
+// a last bit of an integral or a vector flips roundings of the TF32 splits, which moves a converged vector by 1e-8.
 //
 // Bound by the FP64 pipe: the instruction runs at 37 TFLOP/s on this part, the same as scalar fma, but one operand
 // word read from shared memory feeds eight products instead of four or eight registers' worth of broadcasts, so the
@@ -18,9 +18,10 @@
 // as a second phase (6-10 %), four blocks per SM on 64 x 64 tiles (21-25), a fifth warp that only copies (registers
 // spill at two blocks per SM), the copies dealt between the products (the loop outgrows the instruction cache: 9-17).
 //
-// A launch of few tiles is bound by the latency of a slice (copy, barrier, products: 1.3 us), one after another: there
-// eight warps share 64-deep slices of tiles down to 16 x 16. 32 problems of 35 x 35 x (40 x 35): 76 us with four
-// warps, 32-deep slices and 64-row tiles, 48 us so; 64 of 53 x 53 x (40 x 53): 98 -> 83 us.
+// A launch of few tiles is bound by the latency of a slice (copy, barrier, products: 1.3 us), one after another: there the
+// 8 x 8 blocks of tiles down to 16 x 16 are dealt to eight warps, with 64-deep slices. A sigma build of 33,055 CSFs (mixed,
+// its FP64 steps) takes 329 us with four warps and 16-deep slices alone, 264 so; eight warps sharing k, their sums added at
+// the end, took 262, but their sums were not the other form's.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -39,7 +40,8 @@ namespace {
 using tci_dev::DGemmProblem;
 using tci_dev::DGemmSeg;
 
-// Threads of a block: four warps side by side on a tile's columns, or eight sharing k (WK).
+// Threads of a block by work split (WS): four warps side by side on a tile's columns (1), or its 8 x 8 blocks dealt to
+// eight (8).
 constexpr int threads(int wk) { return wk == 1 ? 128 : 256; }
 
 __device__ __forceinline__ void cp_async16(unsigned s, const void* g, int bytes) {
@@ -161,28 +163,28 @@ struct Operand {
   }
 };
 
-// MB: 8-row blocks of a tile.  WK = 1: the four warps share a tile's columns (up to 16 blocks of 8, dealt evenly),
-// 16-deep k slices; WK = 8: eight warps, each takes 8 of every 64-deep slice over the whole tile (up to 4 column
-// blocks), and the eight sums are added in warp order at the end.  Tiles are cut evenly in 8-row / 8-column blocks (a
-// 173-row problem gives 64 + 56 + 56 rows, not 64 + 64 + 45); blocks past the edge are not computed.
-constexpr int NB = 4;  // column blocks of a warp at most
-template <int MB, int WK, Mode AM, Mode BM_>
+// MB: 8-row blocks of a tile.  WS = 1: the four warps share a tile's columns (up to 16 blocks of 8, dealt evenly),
+// 16-deep k slices; WS = 8: the 8 x 8 blocks of a tile (up to 4 columns of them) are dealt to eight warps, 64-deep slices.
+// Tiles are cut evenly in 8-row / 8-column blocks (a 173-row problem gives 64 + 56 + 56 rows, not 64 + 64 + 45); blocks
+// past the edge are not computed.
+constexpr int NB = 4;  // column blocks of a warp (WS = 8: of a tile) at most
+template <int MB, int WS, Mode AM, Mode BM_>
 struct Shape {
-  static constexpr int NT = threads(WK), BK = WK == 1 ? 16 : 64;
-  static constexpr int BM = 8 * MB, BN = 8 * NB * (WK == 1 ? 4 : 1);
+  static constexpr int NT = threads(WS), BK = WS == 1 ? 16 : 64;
+  static constexpr int BM = 8 * MB, BN = 8 * NB * (WS == 1 ? 4 : 1);
   using A = Operand<BM, BK, AM, NT>;
-  using B = Operand<(WK > 1 && BM_ == R16 ? BN + 8 : BN), BK, BM_, NT>;  // room for a shifted row
+  using B = Operand<(WS > 1 && BM_ == R16 ? BN + 8 : BN), BK, BM_, NT>;  // room for a shifted row
   static constexpr int STAGE = A::SIZE + B::SIZE;  // doubles
-  static constexpr int BLOCKS = WK > 1 ? 1 : MB <= 5 || (MB == 6 && AM == K8 && BM_ == R16) ? 3 : 2;  // per SM
+  static constexpr int BLOCKS = WS > 1 ? 1 : MB <= 5 || (MB == 6 && AM == K8 && BM_ == R16) ? 3 : 2;  // per SM
   static constexpr int STG = BLOCKS == 3 ? 3 : 4;
   static constexpr size_t smem = sizeof(double) * (size_t)STAGE * STG;
 };
 
 // ANY: tiles of 1 to MB row blocks in one launch, else of MB or MB - 1.
-template <int MB, int WK, Mode AM, Mode BM_, bool ANY>
-__global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS)) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
+template <int MB, int WS, Mode AM, Mode BM_, bool ANY>
+__global__ void __launch_bounds__(threads(WS), (Shape<MB, WS, AM, BM_>::BLOCKS)) gemm_mma_f64(const DGemmProblem* __restrict__ probs, int nprob,
                                                       const DGemmSeg* __restrict__ segs) {
-  using Sh = Shape<MB, WK, AM, BM_>;
+  using Sh = Shape<MB, WS, AM, BM_>;
   constexpr int NT = Sh::NT, BK = Sh::BK, STG = Sh::STG;
   constexpr bool KB = Sh::B::KROWS;
   extern __shared__ __align__(128) double sm[];
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
   __shared__ int meta_k[STG];  // valid k of the slice; + 256: alpha is not 1; + 512, 1024: shifts of even, odd k
   const int lane = threadIdx.x & 31;
   // rotated: the uneven shares fall on every scheduler in turn
-  const int role = WK == 1 ? ((threadIdx.x >> 5) + blockIdx.x) & 3 : threadIdx.x >> 5;
+  const int role = WS == 1 ? ((threadIdx.x >> 5) + blockIdx.x) & 3 : threadIdx.x >> 5;
   // the problem of this tile (the last with tile_begin <= tile), 32 probes at a time
   const long long tile = blockIdx.x;
   int lo = 0, cnt = nprob;
@@ -206,19 +208,22 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
   const long long rows = tr ? P.N : P.M, cols = tr ? P.M : P.N;
   const int tn = (int)P.tiles_n, t = (int)(tile - P.tile_begin), ti = t / tn, tj = t % tn;
   const int mblk = (int)((rows + 7) >> 3), nblk = (int)((cols + 7) >> 3), tm = (int)(P.trans_c >> 1);
-  const int mq = mblk / tm, mr = mblk % tm, nq = nblk / tn, nr = nblk % tn;
-  const long long m0 = 8ll * (ti * mq + min(ti, mr)), n0 = 8ll * (tj * nq + min(tj, nr));
-  const int mb = mq + (ti < mr ? 1 : 0), nbt = nq + (tj < nr ? 1 : 0);  // mb: MB or MB - 1, ANY: 1 .. MB
+  const int mq = mblk / tm, mr = mblk % tm, nw = nblk / tn, nr = nblk % tn;
+  const long long m0 = 8ll * (ti * mq + min(ti, mr)), n0 = 8ll * (tj * nw + min(tj, nr));
+  const int mb = mq + (ti < mr ? 1 : 0), nbt = nw + (tj < nr ? 1 : 0);  // mb: MB or MB - 1, ANY: 1 .. MB
   const int mrows = (int)min((long long)(8 * mb), rows - m0), ncols = (int)min((long long)(8 * nbt), cols - n0);
   // this warp's column blocks of the tile
-  const int j0 = WK == 1 ? (nbt * role) >> 2 : 0, nb = WK == 1 ? ((nbt * (role + 1)) >> 2) - j0 : nbt;
+  const int j0 = WS == 1 ? (nbt * role) >> 2 : 0, nb = WS == 1 ? ((nbt * (role + 1)) >> 2) - j0 : nbt;
   const int g = lane >> 2, tq = lane & 3;
 
-  double acc[MB][NB][2];
+  // WS = 8: block e = role + 8 q of the tile, row by row, in acc[q][0]
+  constexpr int AR = WS == 1 ? MB : (MB * NB + 7) / 8, AC = WS == 1 ? NB : 1;
+  double acc[AR][AC][2];
 #pragma unroll
-  for (int i = 0; i < MB; ++i)
+  for (int i = 0; i < AR; ++i)
 #pragma unroll
-    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < AC; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int nq = WS == 1 ? 0 : max(0, (mb * nbt - role + 7) >> 3);
 
   // the slices of all segments in table order, copied STG - 1 ahead
   const unsigned sbase = static_cast<unsigned>(__cvta_generic_to_shared(sm));
@@ -276,6 +281,13 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
   // chunks 2 s, 2 s + 1 of a row's 8
   const int f0 = g * BK + 2 * ((tq >> 1) ^ swz(g)) + (tq & 1);
   const int bo = Sh::A::SIZE + (KB ? j0 * 8 + tq * Sh::B::PITCH + g : j0 * 8 * BK);
+  int ao[AR], bq[AR];  // WS = 8: a block's rows and columns in a stage
+#pragma unroll
+  for (int q = 0; q < AR; ++q) {
+    const int e = role + 8 * q;
+    ao[q] = WS == 1 ? 0 : e / nbt * 8 * BK;
+    bq[q] = WS == 1 ? 0 : e % nbt * (KB ? 8 : 8 * BK);
+  }
   int st = 0;
   for (;;) {
     cp_wait<STG - 2>();  // this thread's copies of the slice have landed
@@ -304,15 +316,9 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
           for (int i = 0; i < R; ++i) mma884(acc[i][j][0], acc[i][j][1], a[i], b);
         }
       };
-      if constexpr (WK == 1) {
 #pragma unroll
-        for (int s4 = 0; s4 < BK / 4; ++s4)
-          if (4 * s4 < kc) step(s4);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          if (8 * role + 4 * q < kc) step(2 * role + q);
-      }
+      for (int s4 = 0; s4 < BK / 4; ++s4)
+        if (4 * s4 < kc) step(s4);
     };
     auto bodies = [&](auto rr) {
       if (nb == 4) body(rr, std::integral_constant<int, 4>());
@@ -320,7 +326,34 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
       else if (nb == 2) body(rr, std::integral_constant<int, 2>());
       else if (nb == 1) body(rr, std::integral_constant<int, 1>());
     };
-    if (mb == MB) {
+    if constexpr (WS == 8) {
+      // one chain of fmas per block, four steps' fragments loaded ahead of it (the zeros past the last k add nothing)
+      auto blocks = [&](auto nn) {
+        constexpr int N = decltype(nn)::value;
+#pragma unroll
+        for (int s0 = 0; s0 < BK / 4; s0 += 4) {
+          if (4 * s0 >= kc) break;
+          double a[N][4], b[N][4];
+#pragma unroll
+          for (int q = 0; q < N; ++q)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int fo = (f0 ^ (u << 2)) + (s0 >> 2) * 16;
+              a[q][u] = as[ao[q] + fo];
+              b[q][u] = KB ? bs[(s0 + u) * 4 * Sh::B::PITCH + bq[q]] : bs[bq[q] + fo];
+              if (mk & 256) b[q][u] *= al;
+            }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < N; ++q) mma884(acc[q][0][0], acc[q][0][1], a[q][u], b[q][u]);
+        }
+      };
+      if (AR >= 4 && nq >= 4) blocks(std::integral_constant<int, (AR < 4 ? AR : 4)>());
+      else if (AR >= 3 && nq == 3) blocks(std::integral_constant<int, (AR < 3 ? AR : 3)>());
+      else if (AR >= 2 && nq == 2) blocks(std::integral_constant<int, (AR < 2 ? AR : 2)>());
+      else if (nq >= 1) blocks(std::integral_constant<int, 1>());
+    } else if (mb == MB) {
       bodies(std::integral_constant<int, MB>());
     } else if constexpr (ANY) {
       static_assert(MB == 8, "every height has its body");
@@ -345,7 +378,7 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
     if (c < cols) x[0] = P.beta == 0.0 ? v0 : fma(P.beta, x[0], v0);
     if (c + 1 < cols) x[d] = P.beta == 0.0 ? v1 : fma(P.beta, x[d], v1);
   };
-  if constexpr (WK == 1) {
+  if constexpr (WS == 1) {
 #pragma unroll
     for (int j = 0; j < NB; ++j)
       if (j < nb) {
@@ -354,48 +387,31 @@ __global__ void __launch_bounds__(threads(WK), (Shape<MB, WK, AM, BM_>::BLOCKS))
           if (i < mb) store(i, j, acc[i][j][0], acc[i][j][1]);
       }
   } else {
-    __syncthreads();  // the stages are free
-    double2* red = reinterpret_cast<double2*>(sm);
 #pragma unroll
-    for (int i = 0; i < MB; ++i)
-#pragma unroll
-      for (int j = 0; j < NB; ++j) red[(role * MB * NB + i * NB + j) * 32 + lane] = make_double2(acc[i][j][0], acc[i][j][1]);
-    __syncthreads();
-    for (int e = role; e < MB * NB; e += WK) {
-      const int i = e / NB, j = e % NB;
-      if (i >= mb || j >= nb) continue;
-      double2 v = red[e * 32 + lane];
-#pragma unroll
-      for (int w = 1; w < WK; ++w) {
-        const double2 x = red[(w * MB * NB + e) * 32 + lane];
-        v.x += x.x;
-        v.y += x.y;
-      }
-      store(i, j, v.x, v.y);
-    }
+    for (int q = 0; q < AR; ++q)
+      if (q < nq) store((role + 8 * q) / nbt, (role + 8 * q) % nbt, acc[q][0][0], acc[q][0][1]);
   }
 }
 
-template <int MB, int WK, Mode AM, Mode BM_, bool ANY = false>
+template <int MB, int WS, Mode AM, Mode BM_, bool ANY = false>
 cudaError_t go(const DGemmProblem* probs, int nprob, const DGemmSeg* segs, long long ntiles, cudaStream_t st) {
-  constexpr size_t smem = Shape<MB, WK, AM, BM_>::smem;
-  static_assert(WK == 1 || smem >= sizeof(double2) * WK * MB * NB * 32, "the warps' sums fit the stages");
+  constexpr size_t smem = Shape<MB, WS, AM, BM_>::smem;
   static std::once_flag once[64];  // the attribute, once per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::call_once(once[dev], [&] {
-    cudaFuncSetAttribute(gemm_mma_f64<MB, WK, AM, BM_, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gemm_mma_f64<MB, WS, AM, BM_, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
-  gemm_mma_f64<MB, WK, AM, BM_, ANY><<<(unsigned)ntiles, threads(WK), smem, st>>>(probs, nprob, segs);
+  gemm_mma_f64<MB, WS, AM, BM_, ANY><<<(unsigned)ntiles, threads(WS), smem, st>>>(probs, nprob, segs);
   return cudaGetLastError();
 }
 
 using Go = cudaError_t (*)(const DGemmProblem*, int, const DGemmSeg*, long long, cudaStream_t);
 // one F per row class
-#define TCI_ROWS(F, WK, A, B) \
-  F<1, WK, A, B>, F<2, WK, A, B>, F<3, WK, A, B>, F<4, WK, A, B>, F<5, WK, A, B>, F<6, WK, A, B>, F<7, WK, A, B>, F<8, WK, A, B>
+#define TCI_ROWS(F, WS, A, B) \
+  F<1, WS, A, B>, F<2, WS, A, B>, F<3, WS, A, B>, F<4, WS, A, B>, F<5, WS, A, B>, F<6, WS, A, B>, F<7, WS, A, B>, F<8, WS, A, B>
 #define TCI_PAIR(F, A, B) TCI_ROWS(F, 1, A, B), TCI_ROWS(F, 8, A, B)
 #define TCI_CLASSES(F) \
   TCI_PAIR(F, K16, K16), TCI_PAIR(F, K16, R16), TCI_PAIR(F, K8, K8), TCI_PAIR(F, K8, R16), TCI_PAIR(F, RT8, K8), TCI_PAIR(F, RT8, R16)
@@ -446,12 +462,12 @@ Form form(const DGemmProblem& g, const std::vector<DGemmSeg>& segs) {
   return f;
 }
 
-// Tiles and class of a problem at a largest tile of bmb x bnb blocks; bnb <= NB: the warps share k.
+// Tiles and class of a problem at a largest tile of bmb x bnb blocks; bnb <= NB: the blocks are dealt to eight warps.
 struct Place {
   bool swapped;
   Cut c;
   int cls;
-  double work;  // its largest tile's blocks x its k (k-sharing: four blocks' worth for what a slice costs besides)
+  double work;  // its largest tile's blocks x its k (eight warps: four blocks' worth for what a slice costs besides)
 };
 Place place(const DGemmProblem& g, const Form& f, int bmb, int bnb) {
   Place x;
@@ -500,8 +516,8 @@ Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& seg
   }
   std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return forms[a].k > forms[b].k; });
   // Tile width by the time the fullest SM would need: waves of tiles x the largest tile, the narrower ones at the
-  // rate they were measured at (28 TFLOP/s for 12 blocks, 24 for 8 and 19 for the k-sharing 4 against 30 for 16 on
-  // a launch that fills the chip).  Wide tiles win once there are several waves, narrow and k-sharing ones where a
+  // rate they were measured at (28 TFLOP/s for 12 blocks, 24 for 8 and 19 for the eight warps' 4 against 30 for 16 on
+  // a launch that fills the chip).  Wide tiles win once there are several waves, narrow and dealt ones where a
   // launch would leave SMs idle.
   const double sms = (double)tci_dev::device_sms();
   struct Try {
@@ -534,7 +550,7 @@ Tiles tile(const std::vector<DGemmProblem>& pr, const std::vector<DGemmSeg>& seg
     double n[8] = {}, work[8] = {}, all = 0, longest = 0, apart = 0;
     for (size_t i = 0; i < kinds.size(); ++i) {
       const Place& x = places[i];
-      if (x.cls / 8 != 2 * m) continue;  // eight warps sharing k, or another pair
+      if (x.cls / 8 != 2 * m) continue;  // blocks dealt to eight warps, or another pair
       const double tiles = kinds[i].count * (double)(x.c.tm * x.c.tn);
       n[x.cls % 8] += tiles;
       work[x.cls % 8] = std::max(work[x.cls % 8], x.work);
@@ -575,9 +591,9 @@ cudaError_t launch(const Tables& t, const DGemmSeg* segs, cudaStream_t st) {
 // out: {copies, copies with an address not aligned to the instruction's size, copies from outside the allocation or to
 // outside the slice}.
 namespace {
-template <int MB, int WK, Mode AM, Mode BM_>
+template <int MB, int WS, Mode AM, Mode BM_>
 void copies_of(int which, int nr, long long K, long long ld, long long off, long long len, int64_t* out) {
-  using Sh = Shape<MB, WK, AM, BM_>;
+  using Sh = Shape<MB, WS, AM, BM_>;
   double* const base = reinterpret_cast<double*>((uintptr_t)1 << 40);  // an allocation's alignment; never read
   struct Count {
     int64_t* out;

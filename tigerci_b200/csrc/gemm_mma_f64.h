@@ -9,8 +9,8 @@
 namespace tci_dmma {
 
 // Problems sorted into the kernel's tile classes: six pairs of operand modes (storage order and copy width of the row and
-// the column operand) x two work splits (four warps share a tile's columns, or eight share k where a launch has too few
-// tiles) x one to eight 8-row blocks of a tile; six more for tiles of any height on shared columns, one launch where the
+// the column operand) x two work splits (four warps share a tile's columns, or eight its 8 x 8 blocks where a launch has
+// too few tiles) x one to eight 8-row blocks of a tile; six more for tiles of any height on shared columns, one launch where the
 // heights' own launches would be short.
 constexpr int ROW_CLASSES = 96, CLASSES = ROW_CLASSES + 6;
 struct Tiles {

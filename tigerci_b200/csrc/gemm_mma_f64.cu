@@ -737,6 +737,7 @@ extern "C" int tci_selftest_gemm_f64_group(int64_t device, int64_t nprob, const 
         ok(cudaMemcpy(ds, sg.data(), sizeof(DGemmSeg) * sg.size(), cudaMemcpyHostToDevice));
         ok(cudaMemcpy(dA, A, sizeof(double) * (size_t)ea, cudaMemcpyHostToDevice));
         ok(cudaMemcpy(dB, B, sizeof(double) * (size_t)eb, cudaMemcpyHostToDevice));
+        ok(cudaMemcpy(dC, C, sizeof(double) * (size_t)ec, cudaMemcpyHostToDevice));  // the gaps between the products
         if (rc == TCI_OK) ok(tci_dmma::launch(d, ds, 0));
         ok(cudaDeviceSynchronize());
         if (rc == TCI_OK) ok(cudaMemcpy(C, dC, sizeof(double) * (size_t)ec, cudaMemcpyDeviceToHost));

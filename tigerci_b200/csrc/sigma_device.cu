@@ -1481,8 +1481,9 @@ struct tci_ctx {
     d.tma_ntiles = tiles;
   }
 
-  // At most so many device bytes the compact integral operands of lower_dom take.
-  static i64 dom_operand_bytes(const Plan& P, const tci::LocalSetup& ls) {
+  // At most so many device bytes the compact integral operands of lower_dom take; once: each operand counted once (a
+  // look-up per segment), else once per segment.
+  static i64 dom_operand_bytes(const Plan& P, const tci::LocalSetup& ls, bool once) {
     const i64 n2 = P.n * P.n;
     std::vector<i64> dk2h((size_t)P.nD, -1);
     for (size_t h = 0; h < P.dheads.size(); ++h)
@@ -1496,7 +1497,8 @@ struct tci_ctx {
           const GemmSeg& x = s.gs[(size_t)q];
           const i64 ht = dk2h[(size_t)(g.offC / n2)], hs = dk2h[(size_t)(x.offB / n2)];
           const i64 mt = ls.dh_len[(size_t)ht], ms = ls.dh_len[(size_t)hs];
-          if (mt > 0 && ms > 0 && seen.insert(std::make_tuple((i64)x.a, x.offA, ht, hs)).second) bytes += 8 * mt * (ms + (ms & 1));
+          if (mt <= 0 || ms <= 0 || (once && !seen.insert(std::make_tuple((i64)x.a, x.offA, ht, hs)).second)) continue;
+          bytes += 8 * mt * (ms + (ms & 1));
         }
     }
     return bytes;
@@ -3325,8 +3327,10 @@ int ctx_from_plan(CsfSpace&& sp, Plan&& plan, const double* chol, int64_t device
         if (precision == 0) {
           size_t fr = 0, tot = 0;
           TCI_CUDA(cudaMemGetInfo(&fr, &tot));
-          room = std::max<int64_t>(1, (int64_t)fr - ctx->dom_operand_bytes(P, *ls) - kOperandMargin -
-                                          tci_davidson_bytes(std::max<i64>(1, ctx->n_loc), 1, 50, 0));
+          const int64_t left = (int64_t)fr - kOperandMargin - tci_davidson_bytes(std::max<i64>(1, ctx->n_loc), 1, 50, 0);
+          room = left - ctx->dom_operand_bytes(P, *ls, false);
+          if (room < left / 2) room = left - ctx->dom_operand_bytes(P, *ls, true);
+          room = std::max<int64_t>(1, room);
         }
         const int64_t opts[6] = {precision, 0, kblock, 1, 0, room};
         const int rc = tci_local_create(P.nint, P.n, chol, P.nchol, (int64_t)(ls->heads7.size() / 7), ls->heads7.data(),
